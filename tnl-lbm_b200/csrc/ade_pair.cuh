@@ -76,9 +76,8 @@ __device__ __forceinline__ void ade_pair_write_at(const PairAt& at, const PairSl
 template <typename S, int CUMF, bool ODD>
 __device__ __forceinline__ void ade_pair_update(const StepArgs<typename S::T, float>& a, const CollParams<F2>& p2,
 												const PairSlots& ps, const PairSlots& psd, const AdeArgs<float>& d,
-												const uint8_t* __restrict__ groups, int x, int y, int z)
+												const uint8_t* __restrict__ groups, bool act, int x, int y, int z)
 {
-	bool act = x < a.X && y < a.Y;
 	Site<F2> s;
 	F2 g[7];
 	PairAt at, atd;
@@ -116,9 +115,8 @@ __device__ __forceinline__ void ade_pair_update(const StepArgs<typename S::T, fl
 template <typename S, int CUMF, bool ODD, int MINB>
 __global__ void __launch_bounds__(128, MINB)
 	ade_pair_work_kernel(const StepArgs<typename S::T, float> a, const CollParams<F2> p2, const PairSlots ps,
-						 const PairSlots psd, const AdeArgs<float> d, const uint8_t* __restrict__ groups,
-						 const unsigned* __restrict__ work, const unsigned long long* __restrict__ rest, long long nrest,
-						 int tiles_x)
+						 const PairSlots psd, const PairRows pr, const AdeArgs<float> d, const uint8_t* __restrict__ groups,
+						 const unsigned* __restrict__ work, const unsigned long long* __restrict__ rest, long long nrest)
 {
 	const unsigned w = work[blockIdx.x];
 	if (w & PAIR_WORK_REST) {
@@ -136,9 +134,9 @@ __global__ void __launch_bounds__(128, MINB)
 		ade_site_update<S, COLL_CUM, CUMF, ODD, true, false>(a, d, x, y, z);
 	}
 	else {
-		const unsigned row = w / (unsigned) tiles_x;
-		const int x = (int) (w - row * (unsigned) tiles_x) * 256 + 2 * (int) threadIdx.x;
-		ade_pair_update<S, CUMF, ODD>(a, p2, ps, psd, d, groups, x, (int) (row % (unsigned) a.Y), (int) (row / (unsigned) a.Y));
+		int x, y, z;
+		const bool act = pair_position(pr, w * 128 + threadIdx.x, x, y, z);
+		ade_pair_update<S, CUMF, ODD>(a, p2, ps, psd, d, groups, act, x, y, z);
 	}
 }
 
@@ -210,15 +208,17 @@ cudaError_t ade_pair_step(const StepLaunch& L)
 		*L.blocks_out = (long long) W.nwork * 4;
 	if (L.dry_run)
 		return cudaSuccess;
-	const int tiles_x = ((L.g.X + 1) / 2 + 127) / 128;
+	PairRows pr;
+	if (!make_pair_rows(L.g.X, L.g.Y, L.g.Z, pr))
+		return cudaErrorNotSupported;
 #define LBM_ADE_PAIR(CUMF)                                                                                             \
 	do {                                                                                                               \
 		if (L.odd)                                                                                                     \
 			ade_pair_work_kernel<S, CUMF, true, ADE_PAIR_MINB_ODD>                                                         \
-				<<<grid, block, 0, L.stream>>>(a, p2, ps, psd, d, A->pair_groups, W.work, W.rest, W.nrest, tiles_x);            \
+				<<<grid, block, 0, L.stream>>>(a, p2, ps, psd, pr, d, A->pair_groups, W.work, W.rest, W.nrest);                 \
 		else                                                                                                           \
 			ade_pair_work_kernel<S, CUMF, false, ADE_PAIR_MINB_EVEN>                                                        \
-				<<<grid, block, 0, L.stream>>>(a, p2, ps, psd, d, A->pair_groups, W.work, W.rest, W.nrest, tiles_x);            \
+				<<<grid, block, 0, L.stream>>>(a, p2, ps, psd, pr, d, A->pair_groups, W.work, W.rest, W.nrest);                 \
 	} while (0)
 	switch (L.cum_flags) {
 		case 0:

@@ -146,8 +146,9 @@ struct lbm_lattice
 		const long long tile = (long long) lbm::TILE_MAX_BLOCKS_PER_SM * sms;
 		const dim3 b = block();
 		const long long direct = grid_blocks() * ((b.x * b.y) / 32);
-		// pair step: the two-site grid's warps, or the work list's (4 per item)
-		long long pairs = (long long) (((d.X + 1) / 2 + b.x - 1) / b.x) * ((d.Y + b.y - 1) / b.y) * d.Z * ((b.x * b.y) / 32);
+		// pair step: the warps of the linear pair order, or the work list's (4 per item)
+		const long long threads = b.x * b.y, npairs = (long long) (d.X / 2 + d.X % 2) * d.Y * d.Z;
+		long long pairs = (npairs + threads - 1) / threads * (threads / 32);
 		for (long long nw : pair_nwork)
 			pairs = pairs > 4 * nw ? pairs : 4 * nw;
 		const long long m = tile > direct ? tile : direct;

@@ -615,11 +615,9 @@ int lbm_set_map(lbm_handle h, const uint8_t* map)
 		// GEO_FLUID, all GEO_PERIODIC, or the rest), the sites of the rest
 		// groups in row order (without GEO_NOTHING sites for plain steps, with
 		// them for observation steps, where they give their outputs), and the
-		// work lists: per z plane the chunks of 128 rest sites that start in it,
-		// then the plane's tiles of 256 x-sites that hold a pair group
+		// work lists
 		const int X = h->d.X, Y = h->d.Y, Z = h->d.Z;
 		const int gx = (X + lbm::PAIR_GROUP - 1) / lbm::PAIR_GROUP;
-		const int tiles_x = ((X + 1) / 2 + 127) / 128;
 		std::vector<uint8_t> groups((size_t) gx * Y * Z);
 		std::vector<unsigned long long> rest[2];
 		for (long long row = 0; row < (long long) Y * Z; row++)
@@ -640,29 +638,9 @@ int lbm_set_map(lbm_handle h, const uint8_t* map)
 					}
 			}
 		std::vector<unsigned> work[2];
-		for (int k = 0; k < 2; k++) {
-			const long long nchunks = ((long long) rest[k].size() + 127) / 128;
-			if (nchunks > (long long) (lbm::PAIR_WORK_REST - 1) || (long long) Y * Z * tiles_x >= (long long) lbm::PAIR_WORK_REST)
+		for (int k = 0; k < 2; k++)
+			if (!lbm::build_pair_work(X, Y, Z, groups, rest[k], work[k]))
 				return fail(LBM_ERR_SIZE, "lattice too large for the pair step's work list");
-			long long c = 0;
-			for (int z = 0; z < Z; z++) {
-				// the chunks whose first site lies in plane z, ahead of the plane's
-				// tiles: the slower per-site work starts first and the tiles fill in
-				// around it (duct 26.7 -> 28.3 GLUPS against chunks after the tiles)
-				while (c < nchunks && (long long) (rest[k][(size_t) c * 128] >> 32) / Y <= z)
-					work[k].push_back(lbm::PAIR_WORK_REST | (unsigned) c++);
-				for (int y = 0; y < Y; y++) {
-					const long long row = (long long) z * Y + y;
-					for (int t = 0; t < tiles_x; t++) {
-						bool any = false;
-						for (int g = t * 256 / lbm::PAIR_GROUP; !any && g < gx && g < (t + 1) * 256 / lbm::PAIR_GROUP; g++)
-							any = groups[row * gx + g] != lbm::PAIR_GROUP_REST;
-						if (any)
-							work[k].push_back((unsigned) (row * tiles_x + t));
-					}
-				}
-			}
-		}
 		cudaFree(h->pair_groups);
 		h->pair_groups = nullptr;
 		LBM_CUDA(cudaMalloc(&h->pair_groups, groups.size()));
@@ -1111,14 +1089,16 @@ int lbm_autotune(lbm_handle h, int ntrials)
 	// a collision plugin runs its own one-site or two-site kernels: the tile
 	// and split kernels are not candidates
 	for (auto& c : cands) {
-		if (c[0] > 32 && c[0] / 2 >= h->d.X)
-			continue;  // far wider than the lattice
 		h->bx = c[0];
 		h->by = c[1];
 		if (ensure_partials(h, h->max_step_blocks()))
 			break;
 		for (int k : {(int) lbm::KERNEL_DIRECT, (int) lbm::KERNEL_PAIR}) {
-			if (k == lbm::KERNEL_PAIR && !pair_ok)
+			if (k == lbm::KERNEL_DIRECT && c[0] > 32 && c[0] / 2 >= h->d.X)
+				continue;  // far wider than the lattice
+			// the two-site kernel takes linear blocks of bx * by pairs: one
+			// candidate of each size
+			if (k == lbm::KERNEL_PAIR && (!pair_ok || c[1] != 1))
 				continue;
 			h->kernel = k;
 			// warm-up pair, then timed steps

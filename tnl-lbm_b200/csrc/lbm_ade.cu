@@ -60,9 +60,6 @@ int ade_build_pair(lbm_lattice* h)
 	const uint8_t* fm = h->map_host.data();
 	const uint8_t* am = s->map_host.data();
 	const int gx = (X + PAIR_GROUP - 1) / PAIR_GROUP;
-	const int tiles_x = ((X + 1) / 2 + 127) / 128;
-	if ((long long) Y * Z * tiles_x >= (long long) PAIR_WORK_REST)
-		return 0;
 	std::vector<uint8_t> groups((size_t) gx * Y * Z);
 	std::vector<unsigned long long> rest;
 	for (long long row = 0; row < (long long) Y * Z; row++)
@@ -80,26 +77,9 @@ int ade_build_pair(lbm_lattice* h)
 					if (fm[row * X + x] != GEO_NOTHING || am[row * X + x] != ADE_NOTHING)
 						rest.push_back((unsigned long long) row << 32 | (unsigned) x);
 		}
-	const long long nchunks = ((long long) rest.size() + 127) / 128;
-	if (nchunks >= (long long) PAIR_WORK_REST)
-		return 0;
 	std::vector<unsigned> work;
-	long long c = 0;
-	for (int z = 0; z < Z; z++) {
-		// the plane's rest chunks first, as the flow step's work list
-		while (c < nchunks && (long long) (rest[(size_t) c * 128] >> 32) / Y <= z)
-			work.push_back(PAIR_WORK_REST | (unsigned) c++);
-		for (int y = 0; y < Y; y++) {
-			const long long row = (long long) z * Y + y;
-			for (int t = 0; t < tiles_x; t++) {
-				bool any = false;
-				for (int g = t * 256 / PAIR_GROUP; !any && g < gx && g < (t + 1) * 256 / PAIR_GROUP; g++)
-					any = groups[row * gx + g] != PAIR_GROUP_REST;
-				if (any)
-					work.push_back((unsigned) (row * tiles_x + t));
-			}
-		}
-	}
+	if (!build_pair_work(X, Y, Z, groups, rest, work))
+		return 0;
 	if (work.empty())
 		return 0;
 	cudaError_t e = cudaMalloc(&s->pair_groups, groups.size());

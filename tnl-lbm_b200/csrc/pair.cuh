@@ -22,6 +22,31 @@
 
 namespace lbm {
 
+// Division by an invariant integer with a multiply-high (Granlund and
+// Montgomery, "Division by invariant integers using multiplication", PLDI
+// 1994): for d >= 1, l = ceil(log2 d), m = floor(2^32 (2^l - d) / d) + 1,
+// n / d = (umulhi(m, n) + n) >> l for every n < 2^31.
+struct FastDiv
+{
+	unsigned m;
+	int l;
+	int d;
+};
+
+inline FastDiv make_fast_div(int d)
+{
+	int l = 0;
+	while ((1ll << l) < d)
+		l++;
+	const unsigned long long m = ((1ull << 32) * ((1ull << l) - (unsigned long long) d)) / (unsigned long long) d + 1ull;
+	return FastDiv{(unsigned) m, l, d};
+}
+
+__device__ __forceinline__ unsigned fast_div(unsigned n, const FastDiv& f)
+{
+	return (__umulhi(f.m, n) + n) >> f.l;
+}
+
 // two FP32 lanes
 struct F2
 {
@@ -335,6 +360,10 @@ struct PairAt
 	char* P[3];		   // row (y, x of the first site) in planes z - 1, z, z + 1
 	long long oy[3];   // byte offsets of rows y - 1, y, y + 1 from row y
 	int left, right;   // x offsets (elements) of the pair's outer neighbours, as PairX
+	// ragged rows only: x offset of the first site's right neighbour, 1 or the
+	// wrap of a pair whose second site lies past the row's end
+	int mid;
+	bool single;  // ragged rows only: the pair's second site lies past the row's end
 };
 
 // neighbours of the pair (x, x + 1) of row (y, z) of the population array f
@@ -355,7 +384,21 @@ __device__ __forceinline__ PairAt pair_at_of(char* f, long long E, int sy, int s
 	at.oy[2] = (long long) ((wrap && y == Y - 1) ? -(Y - 1) : 1) * sy * E;
 	at.left = (wrap && x == 0) ? X - 1 : -1;
 	at.right = (wrap && x + 1 == X - 1) ? -(X - 1) : 1;
+	at.mid = 1;
+	at.single = false;
 	return at;
+}
+
+// The last pair of a periodic row of odd width has one site (x = X - 1): its
+// second lane reads within the row (the ghost site x = X, or what the first
+// lane reads), computes along and is never stored.
+__device__ __forceinline__ void pair_ragged(PairAt& at, int x, int X)
+{
+	if (x + 1 == X) {
+		at.single = true;
+		at.mid = -(X - 1);
+		at.right = 0;
+	}
 }
 
 template <typename T>
@@ -366,7 +409,7 @@ __device__ __forceinline__ PairAt pair_at(const StepArgs<T, float>& a, int x, in
 }
 
 // pair_read with the addresses of PairAt / PairSlots
-template <typename S, bool ODD>
+template <typename S, bool ODD, bool RAGGED = false>
 __device__ __forceinline__ void pair_read_at(const PairAt& at, const PairSlots& ps, Site<F2>& s)
 {
 	using T = typename S::T;
@@ -384,6 +427,8 @@ __device__ __forceinline__ void pair_read_at(const PairAt& at, const PairSlots& 
 					s.f[q] = IO::template load2<opp(q)>(c);
 				else if constexpr (cx(q) > 0)
 					s.f[q] = F2(S::template load<opp(q)>(c + at.left), S::template load<opp(q)>(c));
+				else if constexpr (RAGGED)
+					s.f[q] = F2(S::template load<opp(q)>(c + at.mid), S::template load<opp(q)>(c + at.mid + at.right));
 				else
 					s.f[q] = F2(S::template load<opp(q)>(c + 1), S::template load<opp(q)>(c + 1 + at.right));
 			}
@@ -392,11 +437,27 @@ __device__ __forceinline__ void pair_read_at(const PairAt& at, const PairSlots& 
 }
 
 // pair_write with the addresses of PairAt / PairSlots
-template <typename S, bool ODD>
+template <typename S, bool ODD, bool RAGGED = false>
 __device__ __forceinline__ void pair_write_at(const PairAt& at, const PairSlots& ps, const Site<F2>& s)
 {
 	using T = typename S::T;
 	using IO = PairIO<S>;
+	if constexpr (RAGGED)
+		if (at.single) {
+			static_for<27>(
+				[&](auto Qc)
+				{
+					constexpr int q = decltype(Qc)::value;
+					if constexpr (!ODD)
+						S::template store<opp(q)>(reinterpret_cast<T*>(at.P[1] + ps.b[opp(q)]), s.f[q].v.x);
+					else {
+						T* c = reinterpret_cast<T*>(at.P[1 + cz(q)] + at.oy[1 + cy(q)] + ps.b[q]);
+						S::template store<q>(c + (cx(q) == 0 ? 0 : cx(q) > 0 ? at.mid : at.left), s.f[q].v.x);
+					}
+				}
+			);
+			return;
+		}
 	static_for<27>(
 		[&](auto Qc)
 		{
@@ -463,16 +524,53 @@ __device__ __forceinline__ void pair_outputs(const StepArgs<T, float>& a, bool i
 	}
 }
 
-// The update of the pair (x, x + 1) of row (y, z), cumulant collision on two
-// lanes.  Without a map (GENERAL = false) every site is periodic and X is
-// even.  With a map, the lattice rows are cut into groups of PAIR_GROUP sites
+// Pairs of a lattice in linear order: ceil(X / 2) pairs to a row, rows y
+// fastest.  Blocks take consecutive pairs whatever the width of a row is, so
+// that only a launch's last block has idle lanes.  With blocks of 128 pairs of
+// one row X = 300 kept 59 % of the lanes busy and X = 333 65 %, and the idle
+// ones held registers that this latency-bound step lacks.  B200, us per step,
+// blocks of one row -> linear blocks: Taylor-Green 96x96x64 FP32 23.2 -> 18.4,
+// duct 171x45x45 12.7 -> 11.8, 333x85x59 with obstacles (MRT) 61.0 -> 58.7, duct
+// and scalar 100x50x50 16.7 -> 13.1, 512x128x128 FP32 286 -> 288 (runs of one
+// build differ by 2), FP16 225 -> 222.  Odd periodic widths ran the one-site
+// kernel before: 125x97x61 FP32 33.2 -> 28.8, FP16 26.6 -> 24.6.
+struct PairRows
+{
+	FastDiv px, y;	   // division by the pairs of a row and by Y
+	unsigned npairs;  // of the lattice, below 2^31 (make_pair_rows)
+};
+
+// false: more pairs than the linear order numbers
+inline bool make_pair_rows(int X, int Y, int Z, PairRows& pr)
+{
+	const int px = X / 2 + X % 2;
+	const long long n = (long long) px * Y * Z;
+	if (n >= (1ll << 31) - 1024)
+		return false;
+	pr = PairRows{make_fast_div(px), make_fast_div(Y), (unsigned) n};
+	return true;
+}
+
+// first site (x, y, z) of pair p; false past the last pair
+__device__ __forceinline__ bool pair_position(const PairRows& pr, unsigned p, int& x, int& y, int& z)
+{
+	const unsigned row = fast_div(p, pr.px);
+	x = 2 * (int) (p - row * (unsigned) pr.px.d);
+	z = (int) fast_div(row, pr.y);
+	y = (int) (row - (unsigned) z * (unsigned) pr.y.d);
+	return p < pr.npairs;
+}
+
+// The update of the pair (x, x + 1) of row (y, z), collision on two lanes
+// (act: the pair exists).  Without a map (GENERAL = false) every site is
+// periodic; RAGGED: X is odd and the last pair of a row has one site.  With a map, the lattice rows are cut into groups of PAIR_GROUP sites
 // (whole DRAM sectors of every slot row); groups[row * ceil(X / PAIR_GROUP) +
 // x / PAIR_GROUP] is PAIR_GROUP_FLUID or PAIR_GROUP_PERIODIC when every site
 // of the group has that type, and only those groups are updated here; the
 // sites of the other groups (boundaries, obstacles, the lattice ends) take
 // rest_update, one thread per site.  OUT: the macro field and the partial sums
 // of the pair, the warp's sums in slot `slot` of nslots.  Every thread of the
-// warp calls it (threads past the lattice with x >= X).
+// warp calls it.
 template <int COLL, int CUMF>
 struct BuiltinCollision;
 // true for the built-in collisions, false for a collision plugin's struct
@@ -485,12 +583,11 @@ struct is_builtin_collision<BuiltinCollision<COLL, CUMF>> : std::true_type
 {
 };
 
-template <typename S, typename C, bool ODD, bool GENERAL, bool OUT>
+template <typename S, typename C, bool ODD, bool GENERAL, bool OUT, bool RAGGED>
 __device__ __forceinline__ void pair_update(const StepArgs<typename S::T, float>& a, const CollParams<F2>& p2,
-											const PairSlots& ps, const uint8_t* __restrict__ groups, int x, int y, int z,
-											long long slot, long long nslots)
+											const PairSlots& ps, const uint8_t* __restrict__ groups, bool act, int x, int y,
+											int z, long long slot, long long nslots)
 {
-	bool act = x < a.X && y < a.Y;
 	long long site = 0;
 	Site<F2> s;
 	PairAt at;
@@ -515,7 +612,9 @@ __device__ __forceinline__ void pair_update(const StepArgs<typename S::T, float>
 		}
 		else {
 			at = pair_at(a, x, y, z, true);
-			pair_read_at<S, ODD>(at, ps, s);
+			if constexpr (RAGGED)
+				pair_ragged(at, x, a.X);
+			pair_read_at<S, ODD, RAGGED>(at, ps, s);
 		}
 		if (act)
 			density_velocity(s, p2);
@@ -530,7 +629,8 @@ __device__ __forceinline__ void pair_update(const StepArgs<typename S::T, float>
 		return;
 	}
 	else if constexpr (OUT)
-		pair_outputs(a, act, act, site, s, slot, nslots);  // no map: before the collision (fewer live registers)
+		// no map: before the collision (fewer live registers)
+		pair_outputs(a, act, act && !(RAGGED && at.single), site, s, slot, nslots);
 	else if constexpr (!GENERAL || sizeof(typename S::T) == 2 || !is_builtin_collision<C>::value)
 		// keeps the collision after the loads (fewer live registers).  The work
 		// kernel of 32-bit storage with a built-in collision runs without it:
@@ -542,7 +642,7 @@ __device__ __forceinline__ void pair_update(const StepArgs<typename S::T, float>
 	if (!act)
 		return;
 	C::template collision<F2>(s, p2);
-	pair_write_at<S, ODD>(at, ps, s);
+	pair_write_at<S, ODD, RAGGED>(at, ps, s);
 }
 
 // The per-site update of aa_step_kernel for entry i of a host-built site list
@@ -608,33 +708,32 @@ __device__ __forceinline__ void rest_update(const StepArgs<typename S::T, float>
 	aa_write<S, ODD>(a.f, a.sq, base, o, s.f);
 }
 
-// One A-A step of a lattice without a map, two sites per thread: thread
-// (t, y) of the grid owns sites x = 2t and 2t + 1 of row (y, z = blockIdx.z).
-template <typename S, typename C, bool ODD, bool OUT, int MINB>
+// One A-A step of a lattice without a map, two sites per thread: block b takes
+// pairs b T .. b T + T - 1 of the linear order (T = 64 or 128 threads).
+template <typename S, typename C, bool ODD, bool OUT, bool RAGGED, int MINB>
 __global__ void __launch_bounds__(128, MINB) aa_pair_kernel(const StepArgs<typename S::T, float> a, const CollParams<F2> p2,
-															 const PairSlots ps, long long red_slots)
+															 const PairSlots ps, const PairRows pr, long long red_slots)
 {
 	if constexpr (OUT)
 		launch_dependents();
-	const int wpb = (blockDim.x * blockDim.y) >> 5;
-	const long long block = blockIdx.x + (long long) gridDim.x * (blockIdx.y + (long long) gridDim.y * blockIdx.z);
-	const long long slot = block * wpb + ((threadIdx.x + blockDim.x * threadIdx.y) >> 5);
-	pair_update<S, C, ODD, false, OUT>(a, p2, ps, nullptr, 2 * (int) (blockIdx.x * blockDim.x + threadIdx.x),
-										  blockIdx.y * blockDim.y + threadIdx.y, blockIdx.z, slot, red_slots);
+	const long long slot = (long long) blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+	int x, y, z;
+	const bool act = pair_position(pr, blockIdx.x * blockDim.x + threadIdx.x, x, y, z);
+	pair_update<S, C, ODD, false, OUT, RAGGED>(a, p2, ps, nullptr, act, x, y, z, slot, red_slots);
 }
 
 // One A-A step of a lattice with a map in one launch of 128-thread blocks, each
-// taking one item of a host-built work list, in z-plane order: a tile of 256
-// x-sites of one row through pair_update (item = row * tiles_x + tile), or 128
+// taking one item of a host-built work list, in z-plane order: 128 pairs of the
+// linear order through pair_update (item = first pair / 128), or 128
 // entries of the rest-site list through rest_update (item = PAIR_WORK_REST |
 // chunk).  A plane's rest chunks come first and its pair tiles after them, so
 // the rest sites run while the pair tiles around them are in flight and share
 // their DRAM sectors through L2.  Warp w of block b writes partial-sum slot 4 b + w.
 template <typename S, typename C, bool ODD, bool OUT, int MINB>
 __global__ void __launch_bounds__(128, MINB)
-	aa_pair_work_kernel(const StepArgs<typename S::T, float> a, const CollParams<F2> p2, const PairSlots ps,
+	aa_pair_work_kernel(const StepArgs<typename S::T, float> a, const CollParams<F2> p2, const PairSlots ps, const PairRows pr,
 						const uint8_t* __restrict__ groups, const unsigned* __restrict__ work,
-						const unsigned long long* __restrict__ rest, long long nrest, int tiles_x)
+						const unsigned long long* __restrict__ rest, long long nrest)
 {
 	if constexpr (OUT)
 		launch_dependents();
@@ -645,10 +744,9 @@ __global__ void __launch_bounds__(128, MINB)
 		rest_update<S, C, ODD, OUT>(a, rest, nrest, (long long) (w & ~PAIR_WORK_REST) * 128 + threadIdx.x, slot, nslots);
 	}
 	else {
-		const unsigned row = w / (unsigned) tiles_x;
-		const int x = (int) (w - row * (unsigned) tiles_x) * 256 + 2 * (int) threadIdx.x;
-		pair_update<S, C, ODD, true, OUT>(a, p2, ps, groups, x, (int) (row % (unsigned) a.Y), (int) (row / (unsigned) a.Y),
-											 slot, nslots);
+		int x, y, z;
+		const bool act = pair_position(pr, w * 128 + threadIdx.x, x, y, z);
+		pair_update<S, C, ODD, true, OUT, false>(a, p2, ps, groups, act, x, y, z, slot, nslots);
 	}
 }
 
@@ -688,8 +786,8 @@ struct BuiltinCollision
 
 // One A-A step of collision type C (BuiltinCollision, or a collision
 // plugin's struct) through aa_pair_kernel (no map) or aa_pair_work_kernel (a
-// map); cudaErrorNotSupported for periodic lattices of odd width and for
-// storage geometries the two-site accesses cannot align to.
+// map); cudaErrorNotSupported for storage geometries the two-site accesses
+// cannot align to.
 template <typename S, typename C>
 cudaError_t pair_step_with(const StepLaunch& L)
 {
@@ -701,7 +799,8 @@ cudaError_t pair_step_with(const StepLaunch& L)
 	// GEO_NOTHING sites (they output rho = 1, u = 0); a sums-only step runs
 	// the plain list, and the finish kernel adds those sites' rho = 1 each
 	const PairWork& W = L.macro ? L.pair_work_out : L.pair_work;
-	if (general ? (!W.work || !L.pair_groups || W.nwork < 1) : (L.g.X % 2 != 0))
+	PairRows pr;
+	if ((general && (!W.work || !L.pair_groups || W.nwork < 1)) || !make_pair_rows(L.g.X, L.g.Y, L.g.Z, pr))
 		return cudaErrorNotSupported;
 	// 8- and 4-byte alignment of every pair's first site
 	if ((L.g.x0 | L.g.sq | L.g.sy | L.g.sz) & 1)
@@ -728,19 +827,17 @@ cudaError_t pair_step_with(const StepLaunch& L)
 	if (27ll * L.g.sq * (long long) sizeof(T) >= (1ll << 31))
 		return cudaErrorNotSupported;
 	const PairSlots ps = make_pair_slots(L.g.sq, (int) sizeof(T));
-	const dim3 block = general ? dim3(128, 1, 1) : L.block;
-	const int pairs = (L.g.X + 1) / 2;
-	const dim3 grid = general ? dim3((unsigned) W.nwork, 1, 1)
-							  : dim3((pairs + block.x - 1) / block.x, (L.g.Y + block.y - 1) / block.y, L.g.Z);
+	const unsigned threads = general ? 128 : L.block.x * L.block.y;
+	const unsigned grid = general ? (unsigned) W.nwork : (pr.npairs + threads - 1) / threads;
 	// one partial-sum slot per warp
-	const long long red_slots = (long long) grid.x * grid.y * grid.z * ((block.x * block.y) / 32);
+	const long long red_slots = (long long) grid * (threads / 32);
 	if (L.blocks_out)
 		*L.blocks_out = red_slots;
 	if (L.nothing_skipped)
 		*L.nothing_skipped = general && L.partials && !L.macro;
 	if (L.dry_run)
 		return cudaSuccess;
-	const int tiles_x = (pairs + 127) / 128;
+	const bool ragged = L.g.X % 2 != 0;
 	auto launch = [&](auto odd)
 	{
 		constexpr bool ODD = decltype(odd)::value;
@@ -748,15 +845,21 @@ cudaError_t pair_step_with(const StepLaunch& L)
 		if (general) {
 			if (out)
 				aa_pair_work_kernel<S, C, ODD, true, MINB>
-					<<<grid, block, 0, L.stream>>>(a, p2, ps, L.pair_groups, W.work, W.rest, W.nrest, tiles_x);
+					<<<grid, threads, 0, L.stream>>>(a, p2, ps, pr, L.pair_groups, W.work, W.rest, W.nrest);
 			else
 				aa_pair_work_kernel<S, C, ODD, false, MINB>
-					<<<grid, block, 0, L.stream>>>(a, p2, ps, L.pair_groups, W.work, W.rest, W.nrest, tiles_x);
+					<<<grid, threads, 0, L.stream>>>(a, p2, ps, pr, L.pair_groups, W.work, W.rest, W.nrest);
+		}
+		else if (ragged) {
+			if (out)
+				aa_pair_kernel<S, C, ODD, true, true, MINB><<<grid, threads, 0, L.stream>>>(a, p2, ps, pr, red_slots);
+			else
+				aa_pair_kernel<S, C, ODD, false, true, MINB><<<grid, threads, 0, L.stream>>>(a, p2, ps, pr, red_slots);
 		}
 		else if (out)
-			aa_pair_kernel<S, C, ODD, true, MINB><<<grid, block, 0, L.stream>>>(a, p2, ps, red_slots);
+			aa_pair_kernel<S, C, ODD, true, false, MINB><<<grid, threads, 0, L.stream>>>(a, p2, ps, pr, red_slots);
 		else
-			aa_pair_kernel<S, C, ODD, false, MINB><<<grid, block, 0, L.stream>>>(a, p2, ps, red_slots);
+			aa_pair_kernel<S, C, ODD, false, false, MINB><<<grid, threads, 0, L.stream>>>(a, p2, ps, pr, red_slots);
 	};
 	if (L.odd)
 		launch(std::true_type{});
