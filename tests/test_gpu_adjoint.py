@@ -103,6 +103,24 @@ def test_initial_population_gradient_matches_finite_differences(pl, port):
     lat.close()
 
 
+@pytest.mark.parametrize("kind", ["duct", "sym", "periodic"])
+@pytest.mark.parametrize("nsteps,every", [(1, 0), (9, 0), (30, 0), (30, 3), (40, 20)])
+def test_kept_moments_do_not_change_the_gradient(pl, port, kind, nsteps, every):
+    """The last steps' moments kept by the forward pass (as many as the interval
+    leaves room for) against an interval that leaves none (every = 1), and a
+    second backward pass over the same forward pass: the same operations in the
+    same order, bit for bit."""
+    lat, m, f0, force, samples, target, _ = channel(pl, port, pl.STORE_F64, kind, seed=10)
+    run(lat, f0, force, samples, target, nsteps, every=1)
+    want, wp = lat.adjoint_backward(populations=True)
+    run(lat, f0, force, samples, target, nsteps, every=every)
+    for seed in (2.0, 1.0):
+        got, gp = lat.adjoint_backward(seed=seed, populations=True)
+    assert np.max(np.abs(want)) > 0
+    assert np.array_equal(got, want) and np.array_equal(gp, wp)
+    lat.close()
+
+
 def test_checkpoint_interval_does_not_change_the_gradient(pl, port):
     lat, m, f0, force, samples, target, _ = channel(pl, port, pl.STORE_F64, "duct", seed=9)
     N = 21

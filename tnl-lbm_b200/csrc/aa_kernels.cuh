@@ -42,6 +42,31 @@ __device__ __forceinline__ void static_for(F&& f)
 	static_for_impl(std::make_integer_sequence<int, N>{}, f);
 }
 
+// Division by an invariant integer with a multiply-high (Granlund and
+// Montgomery, "Division by invariant integers using multiplication", PLDI
+// 1994): for d >= 1, l = ceil(log2 d), m = floor(2^32 (2^l - d) / d) + 1,
+// n / d = (umulhi(m, n) + n) >> l for every n < 2^31.
+struct FastDiv
+{
+	unsigned m;
+	int l;
+	int d;
+};
+
+inline FastDiv make_fast_div(int d)
+{
+	int l = 0;
+	while ((1ll << l) < d)
+		l++;
+	const unsigned long long m = ((1ull << 32) * ((1ull << l) - (unsigned long long) d)) / (unsigned long long) d + 1ull;
+	return FastDiv{(unsigned) m, l, d};
+}
+
+__device__ __forceinline__ unsigned fast_div(unsigned n, const FastDiv& f)
+{
+	return (__umulhi(f.m, n) + n) >> f.l;
+}
+
 // number of FP64 reduction quantities per block: sum rho, rho*vx, rho*vy,
 // rho*vz, rho*|u|^2 and the count of non-finite densities
 constexpr int NRED = 6;

@@ -30,19 +30,43 @@
 
 namespace lbm {
 
-// resident blocks per SM of the adjoint step (register cap 65536 / (128 n))
+// Resident blocks per SM of the adjoint step (register cap 65536 / (128 n)).  It
+// moves 520 bytes a site (27 FP64 values in and out, 4 moments, the force, the
+// force gradient in and out) and is bound by the latency of its gathers: 64 steps
+// of a 160x48x48 channel backward took 2597 us at 4 blocks, 2512 at 5, 2497 at 6
+// (80 registers, 44 bytes of spills in the odd step), against 6599 when each step
+// read the 27 primal populations, summed direction by direction and ran on rows
+// of 128 threads.
 #ifndef ADJ_STEP_MINB
-#define ADJ_STEP_MINB 4
+#define ADJ_STEP_MINB 6
 #endif
+// and of the primal step with a force field: 64 steps forward (FP32) took
+// 2180 us at 4 blocks, 2207 at 5 (92-112 bytes of spills), 2320 at 6; FP64
+// spills 330 bytes at 4 and runs 3
+#ifndef ADJ_PRIMAL_MINB
+#define ADJ_PRIMAL_MINB 4
+#endif
+template <typename R, bool ODD>
+constexpr int adj_primal_minb()
+{
+	return sizeof(R) == 8 ? 3 : ADJ_PRIMAL_MINB;
+}
 
 template <typename T, typename R>
 struct AdjArgs
 {
 	T* f;			   // primal populations (the step's input, or the state to observe)
 	double* lam;	   // adjoint populations, FP64 whatever the storage, same layout (element strides) as f
+	// density and velocity [4][Z][Y][X] of one step's sites before the collision
+	// (density_velocity): written by the primal step (or null), read by the
+	// adjoint step
+	R* mom;
 	long long sq;
 	int sy, sz, x0;
 	int X, Y, Z;
+	FastDiv dx, dy;	 // division by X and by Y
+	unsigned n;		 // sites
+	int slot[27];	 // byte offsets of lam's 27 slot rows of a lattice row
 	const uint8_t* map;	 // null: every site periodic
 	const R* in_vx;		 // inlet profiles [Z][Y] (GEO_INFLOW) or null
 	const R* in_vy;
@@ -52,8 +76,23 @@ struct AdjArgs
 	CollParams<R> p;
 };
 
-// location of the value that direction q of a site reads (R_q) or writes
-// (W_q) in the A-A step of the given parity
+// Sites are taken in linear order, 128 to a block, whatever the width of a row
+// is: with one row per block column a channel of X = 160 kept 62 % of the lanes
+// busy.  false past the last site.
+template <typename T, typename R>
+__device__ __forceinline__ bool adj_position(const AdjArgs<T, R>& a, long long& site, int& x, int& y, int& z)
+{
+	const unsigned i = blockIdx.x * blockDim.x + threadIdx.x;
+	const unsigned row = fast_div(i, a.dx);
+	x = (int) (i - row * (unsigned) a.X);
+	z = (int) fast_div(row, a.dy);
+	y = (int) (row - (unsigned) z * (unsigned) a.Y);
+	site = i;
+	return i < a.n;
+}
+
+// location of the value that direction q of a site reads (R_q) in the A-A
+// step of the given parity
 template <bool ODD, int q>
 __device__ __forceinline__ long long aa_read_loc(long long sq, long long base, const Offsets& o)
 {
@@ -62,13 +101,54 @@ __device__ __forceinline__ long long aa_read_loc(long long sq, long long base, c
 	else
 		return q * sq + base;
 }
+// Addresses of a site's adjoint values: row pointers of the three z planes
+// around it, the y and x steps from there, and the slots' offsets as constant
+// operands (AdjArgs::slot), so that neither the gather nor the scatter
+// multiplies (as PairAt of pair.cuh)
+struct AdjAt
+{
+	char* P[3];		  // the site in planes z - 1, z, z + 1
+	long long oy[3];  // byte offsets of rows y - 1, y, y + 1
+	int ox[3];		  // and of sites x - 1, x, x + 1
+};
+
+template <typename T, typename R>
+__device__ __forceinline__ AdjAt adj_at(const AdjArgs<T, R>& a, bool wrap, int x, int y, int z)
+{
+	constexpr int E = (int) sizeof(double);
+	const int zm = wrap && z == 0 ? a.Z - 1 : z - 1, zp = wrap && z == a.Z - 1 ? 0 : z + 1;
+	char* const row = reinterpret_cast<char*>(a.lam) + ((long long) (y + 1) * a.sy + a.x0 + x) * E;
+	const long long plane = (long long) a.sz * E;
+	AdjAt at;
+	at.P[0] = row + (zm + 1) * plane;
+	at.P[1] = row + (z + 1) * plane;
+	at.P[2] = row + (zp + 1) * plane;
+	at.oy[0] = (long long) (wrap && y == 0 ? a.Y - 1 : -1) * a.sy * E;
+	at.oy[1] = 0;
+	at.oy[2] = (long long) (wrap && y == a.Y - 1 ? -(a.Y - 1) : 1) * a.sy * E;
+	at.ox[0] = (wrap && x == 0 ? a.X - 1 : -1) * E;
+	at.ox[1] = 0;
+	at.ox[2] = (wrap && x == a.X - 1 ? -(a.X - 1) : 1) * E;
+	return at;
+}
+
+// where direction q of the site is written (its adjoint gathered) and read
+// (its adjoint scattered)
 template <bool ODD, int q>
-__device__ __forceinline__ long long aa_write_loc(long long sq, long long base, const Offsets& o)
+__device__ __forceinline__ double* adj_write_at(const AdjAt& at, const int (&slot)[27])
 {
 	if constexpr (ODD)
-		return q * sq + base + o.x[1 + cx(q)] + o.y[1 + cy(q)] + o.z[1 + cz(q)];
+		return reinterpret_cast<double*>(at.P[1 + cz(q)] + at.oy[1 + cy(q)] + at.ox[1 + cx(q)] + slot[q]);
 	else
-		return opp(q) * sq + base;
+		return reinterpret_cast<double*>(at.P[1] + slot[opp(q)]);
+}
+template <bool ODD, int q>
+__device__ __forceinline__ double* adj_read_at(const AdjAt& at, const int (&slot)[27])
+{
+	if constexpr (ODD)
+		return reinterpret_cast<double*>(at.P[1 - cz(q)] + at.oy[1 - cy(q)] + at.ox[1 - cx(q)] + slot[opp(q)]);
+	else
+		return reinterpret_cast<double*>(at.P[1] + slot[q]);
 }
 
 // collision constants of one site: the per-site force replaces the uniform one
@@ -119,14 +199,14 @@ struct AdjSite
 };
 
 template <typename R>
-__device__ __forceinline__ AdjSite adj_site(const Site<R>& s, const CollParams<R>& p)
+__device__ __forceinline__ AdjSite adj_site(R rho, R vx, R vy, R vz, const CollParams<R>& p)
 {
 	AdjSite m;
-	m.rho = (double) s.rho;
-	m.ir = s.rho == R(0) ? 1.0 : (double) s.ir;
-	m.vx = (double) s.vx;
-	m.vy = (double) s.vy;
-	m.vz = (double) s.vz;
+	m.rho = (double) rho;
+	m.ir = rho == R(0) ? 1.0 : (double) rcp(rho);
+	m.vx = (double) vx;
+	m.vy = (double) vy;
+	m.vz = (double) vz;
 	m.fx = (double) p.fx;
 	m.fy = (double) p.fy;
 	m.fz = (double) p.fz;
@@ -135,51 +215,100 @@ __device__ __forceinline__ AdjSite adj_site(const Site<R>& s, const CollParams<R
 	return m;
 }
 
-// transpose of the SRT update with body force at one site, in place: l <-
-// J^T l, and the force gradient dF += (d out / d F)^T l
-__device__ __forceinline__ void srt_vjp(const AdjSite& m, double* l, double* dF)
+// Transpose of the SRT update with body force at one site: l <- J^T l, and the
+// force gradient dF += (d out / d F)^T l.  With g_q = w_q l_q every sum over the
+// directions is one of the moments T_abc = sum_q g_q cx^a cy^b cz^c of order
+// <= 3 (c^3 = c), and the weights factorise over the axes (2/3 and 1/6), so the
+// 27 values are reduced line by line (three operations a line, 1/6 of each axis
+// left to the end) and the rest is algebra on 17 numbers: about 240 FP64
+// operations a site instead of about 1000 direction by direction.  The new
+// value of direction j goes to put(j, value).
+template <typename Put>
+__device__ __forceinline__ void srt_vjp(const AdjSite& m, const double* l, double* dF, Put&& put)
 {
 	const double rho = m.rho, ir = m.ir;
 	const double vx = m.vx, vy = m.vy, vz = m.vz;
-	const double usq = vx * vx + vy * vy + vz * vz;
 	const double it = m.inv_tau, k = m.srt_force;
-	double A = 0, bx = 0, by = 0, bz = 0, hx = 0, hy = 0, hz = 0;
+	// moments, the powers of cx, cy and cz in turn
+	double M[27];
 	static_for<27>(
 		[&](auto Qc)
 		{
 			constexpr int q = decltype(Qc)::value;
-			const double feq = eq_second<q>(rho, vx, vy, vz, usq);
-			const double S = 3.0 * ((cx(q) - vx) * m.fx + (cy(q) - vy) * m.fy + (cz(q) - vz) * m.fz) * ir;
-			const double lq = l[q];
-			A += lq * feq;
-			// d feq / d u weighted by (it + k S)
-			add_dfeq_du<q>(lq * (it + k * S), rho, vx, vy, vz, bx, by, bz);
-			// k feq dS/du = -3 k feq F / rho ; k feq dS/dF_a = 3 k feq (c_a - u_a) / rho
-			const double lf = lq * feq;
-			hx += lf * (cx(q) - vx);
-			hy += lf * (cy(q) - vy);
-			hz += lf * (cz(q) - vz);
+			M[ci(cx(q) + 1, cy(q) + 1, cz(q) + 1)] = l[q];
 		}
 	);
-	// sum_q l_q feq_q, used by the density derivative and the dS/du term
-	const double sum_lf = A;
-	A = it * sum_lf * ir;
-	bx -= 3.0 * k * sum_lf * m.fx * ir;
-	by -= 3.0 * k * sum_lf * m.fy * ir;
-	bz -= 3.0 * k * sum_lf * m.fz * ir;
+	auto line = [](double& a, double& b, double& c)
+	{
+		const double s = c + a, d = c - a;
+		a = s + 4.0 * b;
+		b = d;
+		c = s;
+	};
+#pragma unroll
+	for (int j = 0; j < 3; j++)
+#pragma unroll
+		for (int i = 0; i < 3; i++)
+			line(M[ci(0, j, i)], M[ci(1, j, i)], M[ci(2, j, i)]);
+#pragma unroll
+	for (int j = 0; j < 3; j++)
+#pragma unroll
+		for (int i = 0; i < 3; i++)
+			line(M[ci(j, 0, i)], M[ci(j, 1, i)], M[ci(j, 2, i)]);
+#pragma unroll
+	for (int j = 0; j < 3; j++)
+#pragma unroll
+		for (int i = 0; i < 3; i++)
+			line(M[ci(j, i, 0)], M[ci(j, i, 1)], M[ci(j, i, 2)]);
+	const double w = 1.0 / 216.0;
+	const double T000 = w * M[ci(0, 0, 0)], T100 = w * M[ci(1, 0, 0)], T010 = w * M[ci(0, 1, 0)], T001 = w * M[ci(0, 0, 1)];
+	const double T200 = w * M[ci(2, 0, 0)], T020 = w * M[ci(0, 2, 0)], T002 = w * M[ci(0, 0, 2)];
+	const double T110 = w * M[ci(1, 1, 0)], T101 = w * M[ci(1, 0, 1)], T011 = w * M[ci(0, 1, 1)];
+	const double T210 = w * M[ci(2, 1, 0)], T201 = w * M[ci(2, 0, 1)], T120 = w * M[ci(1, 2, 0)], T021 = w * M[ci(0, 2, 1)];
+	const double T102 = w * M[ci(1, 0, 2)], T012 = w * M[ci(0, 1, 2)], T111 = w * M[ci(1, 1, 1)];
+	// second moments contracted with u, and third moments contracted with u once
+	const double ux = vx * T200 + vy * T110 + vz * T101;
+	const double uy = vx * T110 + vy * T020 + vz * T011;
+	const double uz = vx * T101 + vy * T011 + vz * T002;
+	const double U200 = vx * T100 + vy * T210 + vz * T201, U020 = vx * T120 + vy * T010 + vz * T021;
+	const double U002 = vx * T102 + vy * T012 + vz * T001, U110 = vx * T210 + vy * T120 + vz * T111;
+	const double U101 = vx * T201 + vy * T111 + vz * T102, U011 = vx * T111 + vy * T021 + vz * T012;
+	const double e0 = 1.0 - 1.5 * (vx * vx + vy * vy + vz * vz);
+	// sum_q l_q feq_q and sum_q l_q feq_q (c_q - u)
+	const double u1 = vx * T100 + vy * T010 + vz * T001;
+	const double sum_lf = rho * (e0 * T000 + 3.0 * u1 + 4.5 * (vx * ux + vy * uy + vz * uz));
+	const double hx = rho * (e0 * T100 + 3.0 * ux + 4.5 * (vx * U200 + vy * U110 + vz * U101)) - vx * sum_lf;
+	const double hy = rho * (e0 * T010 + 3.0 * uy + 4.5 * (vx * U110 + vy * U020 + vz * U011)) - vy * sum_lf;
+	const double hz = rho * (e0 * T001 + 3.0 * uz + 4.5 * (vx * U101 + vy * U011 + vz * U002)) - vz * sum_lf;
+	// sum_q l_q (1/tau + k S_q) d feq_q / du, S_q = 3 (c_q - u).F / rho and
+	// d feq_q / du = w_q rho ((3 + 9 c.u) c - 3 u), less the part of dS/du
+	const double t = 3.0 * k * ir;
+	const double gx = t * m.fx, gy = t * m.fy, gz = t * m.fz;
+	const double al = it - (gx * vx + gy * vy + gz * vz);
+	const double g1 = al * T000 + (gx * T100 + gy * T010 + gz * T001);
+	const double bx = rho * (3.0 * (al * T100 + (gx * T200 + gy * T110 + gz * T101) - vx * g1)
+							 + 9.0 * (al * ux + gx * U200 + gy * U110 + gz * U101)) - sum_lf * gx;
+	const double by = rho * (3.0 * (al * T010 + (gx * T110 + gy * T020 + gz * T011) - vy * g1)
+							 + 9.0 * (al * uy + gx * U110 + gy * U020 + gz * U011)) - sum_lf * gy;
+	const double bz = rho * (3.0 * (al * T001 + (gx * T101 + gy * T011 + gz * T002) - vz * g1)
+							 + 9.0 * (al * uz + gx * U101 + gy * U011 + gz * U002)) - sum_lf * gz;
+	// the second pass reads l from memory again: held since the first it would
+	// take 54 registers
+	asm volatile("" ::: "memory");
 	const double omit = 1.0 - it;
+	const double Bx = bx * ir, By = by * ir, Bz = bz * ir;
+	const double A = it * sum_lf * ir - (Bx * vx + By * vy + Bz * vz);
 	static_for<27>(
 		[&](auto Qc)
 		{
 			constexpr int j = decltype(Qc)::value;
-			l[j] = omit * l[j] + A + (bx * (cx(j) - vx) + by * (cy(j) - vy) + bz * (cz(j) - vz)) * ir;
+			put(Qc, omit * l[j] + (A + cx(j) * Bx + cy(j) * By + cz(j) * Bz));
 		}
 	);
 	// d out / d F: through u (du/dF = 1 / (2 rho)) and through S directly
-	const double half_ir = 0.5 * ir, three_k_ir = 3.0 * k * ir;
-	dF[0] += bx * half_ir + three_k_ir * hx;
-	dF[1] += by * half_ir + three_k_ir * hy;
-	dF[2] += bz * half_ir + three_k_ir * hz;
+	dF[0] += 0.5 * Bx + t * hx;
+	dF[1] += 0.5 * By + t * hy;
+	dF[2] += 0.5 * Bz + t * hz;
 }
 
 // transpose of out = feq(1, u(f)) (GEO_OUTFLOW_EQ), in place
@@ -245,16 +374,19 @@ __device__ __forceinline__ void symmetry_vjp(double* l, int axis, int side)
 // Primal A-A step with SRT collision and a per-site force: the per-site code
 // of aa_step_kernel (GENERAL, COLL_SRT) with the site's force in place of the
 // uniform one.  With a uniform force field it is the production SRT step.
+// With a.mom the sites' density and velocity before the collision are kept:
+// all that the adjoint of the step needs of its primal input (16 bytes a site in
+// FP32 where the populations are 108).
 template <typename S, bool ODD>
-__global__ void __launch_bounds__(128) adj_primal_kernel(const AdjArgs<typename S::T, typename S::R> a)
+__global__ void __launch_bounds__(128, adj_primal_minb<typename S::R, ODD>())
+	adj_primal_kernel(const AdjArgs<typename S::T, typename S::R> a)
 {
 	using R = typename S::R;
-	const int x = blockIdx.x * blockDim.x + threadIdx.x;
-	const int y = blockIdx.y, z = blockIdx.z;
-	if (x >= a.X)
+	int x, y, z;
+	long long site;
+	if (!adj_position(a, site, x, y, z))
 		return;
-	const long long nsites = (long long) a.X * a.Y * a.Z;
-	const long long site = ((long long) z * a.Y + y) * a.X + x;
+	const long long nsites = a.n;
 	const uint8_t geo = a.map ? a.map[site] : (uint8_t) GEO_PERIODIC;
 	if (geo == GEO_NOTHING)
 		return;
@@ -268,64 +400,79 @@ __global__ void __launch_bounds__(128) adj_primal_kernel(const AdjArgs<typename 
 	const Offsets o = neighbour_offsets(geo == GEO_PERIODIC, x, y, z, a.X, a.Y, a.Z, a.sy, a.sz);
 	Site<R> s;
 	aa_read<S, ODD>(a.f, a.sq, base, o, s.f);
-	if (apply_boundary(s, geo, sa, z, y))
+	R rho_in = R(1);
+	if (geo == GEO_OUTFLOW_EQ) {  // apply_boundary replaces the density
+		density_velocity(s, sa.p);
+		rho_in = s.rho;
+	}
+	const bool coll = apply_boundary(s, geo, sa, z, y);
+	if (a.mom) {
+		a.mom[site] = geo == GEO_OUTFLOW_EQ ? rho_in : s.rho;
+		a.mom[nsites + site] = s.vx;
+		a.mom[2 * nsites + site] = s.vy;
+		a.mom[3 * nsites + site] = s.vz;
+	}
+	if (coll)
 		collide<R, COLL_SRT, 0>(s, sa.p);
 	aa_write<S, ODD>(a.f, a.sq, base, o, s.f);
 }
 
 // Adjoint of one A-A step: lam (adjoint of the step's output) is replaced in
-// place by the adjoint of its input, with f the step's primal input; grad
-// accumulates the force gradient of this step.  The adjoint values of a site
-// are gathered from its write locations, transformed in place in FP64 and
-// scattered to its read locations; the addresses are formed again for the
-// scatter instead of being kept in registers across the transform.  Blocks of
-// 128 threads (the shared array has one row per thread).
-template <typename S, bool ODD>
-__global__ void __launch_bounds__(128, ADJ_STEP_MINB) adj_step_kernel(const AdjArgs<typename S::T, typename S::R> a)
+// place by the adjoint of its input, with mom the moments of the step's primal
+// input; grad accumulates the force gradient of this step.  The adjoint values
+// of a site are gathered from its write locations, transformed in FP64 and
+// scattered to its read locations.  Blocks of 128 threads (the shared array
+// has one row per thread).
+template <typename T, typename R, bool ODD>
+__global__ void __launch_bounds__(128, ADJ_STEP_MINB) adj_step_kernel(const AdjArgs<T, R> a)
 {
-	using R = typename S::R;
-	const int x = blockIdx.x * blockDim.x + threadIdx.x;
-	const int y = blockIdx.y, z = blockIdx.z;
-	if (x >= a.X)
+	int x, y, z;
+	long long site;
+	if (!adj_position(a, site, x, y, z))
 		return;
-	const long long nsites = (long long) a.X * a.Y * a.Z;
-	const long long site = ((long long) z * a.Y + y) * a.X + x;
+	const long long nsites = a.n;
 	const uint8_t geo = a.map ? a.map[site] : (uint8_t) GEO_PERIODIC;
 	if (geo == GEO_NOTHING)
 		return;
-	const long long base = (long long) (z + 1) * a.sz + (long long) (y + 1) * a.sy + a.x0 + x;
 	// the site's 27 adjoint values live in shared memory (27 doubles per
 	// thread, an odd stride: no bank conflicts beyond the two wavefronts of a
 	// 64-bit access), not in registers: 54 registers fewer per thread and so
 	// more resident warps for this memory-bound step
 	__shared__ double lsh[128 * 27];
 	double* const l = lsh + threadIdx.x * 27;
-	// the primal populations of the sites whose transpose needs the moments
-	// are loaded before the adjoint values, so that both sets of loads are in
-	// flight together
-	const bool primal = geo != GEO_WALL && geo != GEO_INFLOW && !(geo >= GEO_SYM_TOP && geo <= GEO_SYM_FRONT);
-	Site<R> s;
-	{
-		const Offsets o = neighbour_offsets(geo == GEO_PERIODIC, x, y, z, a.X, a.Y, a.Z, a.sy, a.sz);
-		// the adjoint values go straight to shared memory (asynchronous copies,
-		// no registers), and the primal loads are in flight with them
-		static_for<27>(
-			[&](auto Qc)
-			{
-				constexpr int q = decltype(Qc)::value;
-				copy8_async(l + q, a.lam + aa_write_loc<ODD, q>(a.sq, base, o));
-			}
-		);
-		asm volatile("cp.async.commit_group;" ::: "memory");
-		if (primal)
-			aa_read<S, ODD>(a.f, a.sq, base, o, s.f);
-		// each thread reads only its own row of lsh: the wait makes this
-		// thread's copies visible to it, no block barrier is needed
-		asm volatile("cp.async.wait_group 0;" ::: "memory");
-	}
+	const bool fluid = geo == GEO_FLUID || geo == GEO_PERIODIC;
+	R mom[4] = {R(1), R(0), R(0), R(0)};
+	AdjAt at = adj_at(a, geo == GEO_PERIODIC, x, y, z);
+	// the adjoint values go straight to shared memory (asynchronous copies,
+	// no registers), and the moments' loads are in flight with them
+	static_for<27>(
+		[&](auto Qc)
+		{
+			constexpr int q = decltype(Qc)::value;
+			copy8_async(l + q, adj_write_at<ODD, q>(at, a.slot));
+		}
+	);
+	asm volatile("cp.async.commit_group;" ::: "memory");
+	if (fluid || geo == GEO_OUTFLOW_EQ)
+#pragma unroll
+		for (int i = 0; i < 4; i++)
+			mom[i] = a.mom[i * nsites + site];
+	const CollParams<R> p = site_params(a, site, nsites);
+	// each thread reads only its own row of lsh: the wait makes this
+	// thread's copies visible to it, no block barrier is needed
+	asm volatile("cp.async.wait_group 0;" ::: "memory");
+	// the scatter's 27 addresses are formed anew from here, not kept since the
+	// gather
+#pragma unroll
+	for (int i = 0; i < 3; i++)
+		asm volatile("" : "+l"(at.P[i]));
 	double dF[3] = {0, 0, 0};
-	switch (geo) {
-		case GEO_WALL:
+	auto put = [&](auto Qc, double v) { *adj_read_at<ODD, decltype(Qc)::value>(at, a.slot) = v; };
+	const AdjSite m = adj_site(mom[0], mom[1], mom[2], mom[3], p);
+	if (fluid)
+		srt_vjp(m, l, dF, put);
+	else {
+		if (geo == GEO_WALL)
 			// full-way bounce-back swaps opposite directions: its transpose too
 			static_for<13>(
 				[&](auto Qc)
@@ -336,8 +483,7 @@ __global__ void __launch_bounds__(128, ADJ_STEP_MINB) adj_step_kernel(const AdjA
 					l[opp(q)] = t;
 				}
 			);
-			break;
-		case GEO_INFLOW:
+		else if (geo == GEO_INFLOW)
 			static_for<27>(
 				[&](auto Qc)
 				{
@@ -345,37 +491,14 @@ __global__ void __launch_bounds__(128, ADJ_STEP_MINB) adj_step_kernel(const AdjA
 					l[q] = 0.0;
 				}
 			);
-			break;
-		case GEO_SYM_TOP:
-		case GEO_SYM_BOTTOM:
-		case GEO_SYM_LEFT:
-		case GEO_SYM_RIGHT:
-		case GEO_SYM_BACK:
-		case GEO_SYM_FRONT: {
+		else if (geo >= GEO_SYM_TOP && geo <= GEO_SYM_FRONT) {
 			const int axis = geo <= GEO_SYM_BOTTOM ? 2 : (geo <= GEO_SYM_RIGHT ? 0 : 1);
 			const int side = (geo == GEO_SYM_TOP || geo == GEO_SYM_RIGHT || geo == GEO_SYM_FRONT) ? -1 : 1;
 			symmetry_vjp(l, axis, side);
-			break;
 		}
-		default: {	// FLUID, PERIODIC, OUTFLOW_EQ: need the primal moments
-			const CollParams<R> p = site_params(a, site, nsites);
-			density_velocity(s, p);
-			const AdjSite m = adj_site(s, p);
-			if (geo == GEO_OUTFLOW_EQ)
-				outflow_eq_vjp(m, l, dF);
-			else
-				srt_vjp(m, l, dF);
-		}
-	}
-	{
-		const Offsets o = neighbour_offsets(geo == GEO_PERIODIC, x, y, z, a.X, a.Y, a.Z, a.sy, a.sz);
-		static_for<27>(
-			[&](auto Qc)
-			{
-				constexpr int q = decltype(Qc)::value;
-				a.lam[aa_read_loc<ODD, q>(a.sq, base, o)] = l[q];
-			}
-		);
+		else
+			outflow_eq_vjp(m, l, dF);
+		static_for<27>([&](auto Qc) { put(Qc, l[decltype(Qc)::value]); });
 	}
 	if (a.grad && a.force && (dF[0] != 0.0 || dF[1] != 0.0 || dF[2] != 0.0)) {
 		a.grad[site] += dF[0];

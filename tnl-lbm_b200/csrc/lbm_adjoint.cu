@@ -3,13 +3,21 @@
 // A-A steps with the SRT collision, with respect to a per-site body force
 // field and to the initial populations.
 //
-// Memory: sqrt(N)-style checkpointing.  The forward pass keeps the population
-// array every K steps (ceil(N/K) checkpoints) and the final state.  The
-// backward pass walks the segments from the last to the first: it restores
-// the segment's checkpoint, recomputes and keeps the K states of the segment,
-// and runs the K adjoint steps backwards through them.  Peak memory is
-// (ceil(N/K) + K + 2) population arrays; K = sqrt(N) minimises it, and the
-// cost is two primal steps and one adjoint step per step.
+// Memory: sqrt(N)-style checkpointing.  The adjoint of a step needs the density
+// and velocity of the step's sites and nothing else of its primal input: 4
+// values a site where the populations are 27.  The forward pass keeps those
+// moments of its last steps (kept_steps), the population array at the start of
+// every segment of K steps before them, and the final state.  The backward pass
+// runs the adjoint steps whose moments are kept, then walks the remaining
+// segments from the last to the first: it restores the segment's checkpoint,
+// recomputes its steps and their moments in one working array, and runs the
+// adjoint steps backwards through them.  Peak memory is below (ceil(N/K) + K +
+// 2) population arrays, a forward pass alone takes at most 2 ceil(N/K) + 1;
+// K = sqrt(N) minimises it.
+//
+// On a 160x48x48 channel (FP32 primal, 64 steps, K = 8; B200) forward and
+// backward took 8.9 ms with the populations of a segment kept (a copy ahead of
+// each recomputed step, 612 bytes a site and adjoint step), now 4.2 (520 bytes).
 //
 // The reference's adjoint (sim_adjoint/sim_adjoint.cu with D3Q27_SRT_ADJOINT,
 // col_srt_adjoint.h) iterates a steady adjoint problem about a frozen primal
@@ -20,7 +28,6 @@
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
-#include <set>
 #include <vector>
 
 #include <cuda_runtime.h>
@@ -37,7 +44,13 @@ struct AdjointState
 	double* force = nullptr;	 // [3][Z][Y][X]
 	std::vector<void*> ckpt;
 	void* final_state = nullptr;
-	std::vector<void*> seg;
+	void* work = nullptr;	 // the segment being recomputed
+	// moments [step][4][Z][Y][X], compute type: of the last `kept` steps of this
+	// run (forward pass), and of the segment being recomputed (backward pass)
+	void* kept_mom = nullptr;
+	void* seg_mom = nullptr;
+	size_t kept_bytes = 0, seg_bytes = 0;  // their capacities
+	long long kept = 0;
 	double* lam = nullptr;	 // FP64, the element strides of the population array
 	double* grad = nullptr;	 // [3][Z][Y][X]
 	long long* samples = nullptr;
@@ -60,8 +73,9 @@ void adjoint_free(AdjointState* a)
 	for (void* p : a->ckpt)
 		cudaFree(p);
 	cudaFree(a->final_state);
-	for (void* p : a->seg)
-		cudaFree(p);
+	cudaFree(a->work);
+	cudaFree(a->kept_mom);
+	cudaFree(a->seg_mom);
 	cudaFree(a->lam);
 	cudaFree(a->grad);
 	cudaFree(a->samples);
@@ -114,18 +128,66 @@ lbm::AdjArgs<typename S::T, typename S::R> make_args(lbm_handle h, void* f, void
 	a.force = h->adjoint->force;
 	a.grad = grad;
 	a.p = lbm::make_coll_params<R>(h->p);
+	a.dx = lbm::make_fast_div(h->d.X);
+	a.dy = lbm::make_fast_div(h->d.Y);
+	a.n = (unsigned) h->sites();
+	for (int q = 0; q < 27; q++)
+		a.slot[q] = (int) (q * h->g.sq * (long long) sizeof(double));
 	return a;
 }
 
-dim3 site_grid(lbm_handle h)
+unsigned site_grid(lbm_handle h)
 {
-	return dim3((unsigned) ((h->d.X + 127) / 128), (unsigned) h->d.Y, (unsigned) h->d.Z);
+	return (unsigned) ((h->sites() + 127) / 128);
+}
+
+// bytes of one step's moments
+size_t moments_bytes(lbm_handle h)
+{
+	return (size_t) 4 * h->sites() * h->ops->compute_size;
+}
+// slot k of the kept or the recomputed moments
+void* moments_of(lbm_handle h, void* mom, long long k)
+{
+	return (char*) mom + (size_t) k * moments_bytes(h);
+}
+
+// The last steps whose moments the forward pass keeps instead of leaving them to
+// be recomputed: as many as fit in the room that a segment's populations would
+// take less a segment's moments, and in that of all checkpoints (a run that
+// never goes backward, with one checkpoint, stays small).
+long long kept_steps(lbm_handle h, long long nsteps, long long every)
+{
+	const double per_array = (double) h->pop_bytes / (double) moments_bytes(h);
+	const long long nckpt = (nsteps + every - 1) / every;
+	long long kept = (long long) ((double) (every - 1) * per_array) - every;
+	const long long most = (long long) ((double) nckpt * per_array);
+	kept = kept < most ? kept : most;
+	return kept < 0 ? 0 : (kept < nsteps ? kept : nsteps);
+}
+
+// grows a device buffer; false when the device has no room (the buffer is then empty)
+bool ensure_bytes(void*& p, size_t& cap, size_t bytes)
+{
+	if (bytes <= cap)
+		return true;
+	cudaFree(p);
+	p = nullptr;
+	cap = 0;
+	if (cudaMalloc(&p, bytes) != cudaSuccess) {
+		cudaGetLastError();	 // reported by the caller
+		p = nullptr;
+		return false;
+	}
+	cap = bytes;
+	return true;
 }
 
 template <typename S>
-cudaError_t primal_step(lbm_handle h, void* f, long long n)
+cudaError_t primal_step(lbm_handle h, void* f, long long n, void* mom)
 {
-	const auto a = make_args<S>(h, f, nullptr, nullptr);
+	auto a = make_args<S>(h, f, nullptr, nullptr);
+	a.mom = (typename S::R*) mom;
 	if ((h->adjoint->it0 + n) & 1)
 		lbm::adj_primal_kernel<S, true><<<site_grid(h), 128, 0, h->stream>>>(a);
 	else
@@ -134,14 +196,17 @@ cudaError_t primal_step(lbm_handle h, void* f, long long n)
 }
 
 template <typename S>
-cudaError_t adjoint_step(lbm_handle h, void* f, long long n)
+cudaError_t adjoint_step(lbm_handle h, long long n, void* mom)
 {
+	using T = typename S::T;
+	using R = typename S::R;
 	auto* st = h->adjoint;
-	const auto a = make_args<S>(h, f, st->lam, st->grad);
+	auto a = make_args<S>(h, nullptr, st->lam, st->grad);
+	a.mom = (R*) mom;
 	if ((st->it0 + n) & 1)
-		lbm::adj_step_kernel<S, true><<<site_grid(h), 128, 0, h->stream>>>(a);
+		lbm::adj_step_kernel<T, R, true><<<site_grid(h), 128, 0, h->stream>>>(a);
 	else
-		lbm::adj_step_kernel<S, false><<<site_grid(h), 128, 0, h->stream>>>(a);
+		lbm::adj_step_kernel<T, R, false><<<site_grid(h), 128, 0, h->stream>>>(a);
 	return cudaGetLastError();
 }
 
@@ -165,10 +230,11 @@ int forward_typed(lbm_handle h)
 {
 	auto* st = h->adjoint;
 	const size_t pb = h->pop_bytes;
+	const long long first_kept = st->nsteps - st->kept;
 	for (long long n = 0; n < st->nsteps; n++) {
-		if (n % st->every == 0)
+		if (n < first_kept && n % st->every == 0)
 			ADJ_CUDA(cudaMemcpyAsync(st->ckpt[(size_t) (n / st->every)], h->g.f, pb, cudaMemcpyDeviceToDevice, h->stream));
-		ADJ_CUDA(primal_step<S>(h, h->g.f, n));
+		ADJ_CUDA(primal_step<S>(h, h->g.f, n, n < first_kept ? nullptr : moments_of(h, st->kept_mom, n - first_kept)));
 	}
 	ADJ_CUDA(cudaMemcpyAsync(st->final_state, h->g.f, pb, cudaMemcpyDeviceToDevice, h->stream));
 	ADJ_CUDA(objective<S>(h, false, 0.0));
@@ -196,17 +262,17 @@ int backward_typed(lbm_handle h, double seed)
 	ADJ_CUDA(cudaMemsetAsync(st->grad, 0, sizeof(double) * 3 * h->sites(), h->stream));
 	ADJ_CUDA(objective<S>(h, true, seed));
 	const size_t pb = h->pop_bytes;
-	const long long nseg = st->nckpt;
-	for (long long s = nseg - 1; s >= 0; s--) {
+	const long long first_kept = st->nsteps - st->kept;
+	for (long long n = st->nsteps - 1; n >= first_kept; n--)
+		ADJ_CUDA(adjoint_step<S>(h, n, moments_of(h, st->kept_mom, n - first_kept)));
+	for (long long s = st->nckpt - 1; s >= 0; s--) {
 		const long long n0 = s * st->every;
-		const long long n1 = n0 + st->every < st->nsteps ? n0 + st->every : st->nsteps;
-		ADJ_CUDA(cudaMemcpyAsync(st->seg[0], st->ckpt[(size_t) s], pb, cudaMemcpyDeviceToDevice, h->stream));
-		for (long long i = 1; i < n1 - n0; i++) {
-			ADJ_CUDA(cudaMemcpyAsync(st->seg[(size_t) i], st->seg[(size_t) (i - 1)], pb, cudaMemcpyDeviceToDevice, h->stream));
-			ADJ_CUDA(primal_step<S>(h, st->seg[(size_t) i], n0 + i - 1));
-		}
+		const long long n1 = n0 + st->every < first_kept ? n0 + st->every : first_kept;
+		ADJ_CUDA(cudaMemcpyAsync(st->work, st->ckpt[(size_t) s], pb, cudaMemcpyDeviceToDevice, h->stream));
+		for (long long n = n0; n < n1; n++)
+			ADJ_CUDA(primal_step<S>(h, st->work, n, moments_of(h, st->seg_mom, n - n0)));
 		for (long long n = n1 - 1; n >= n0; n--)
-			ADJ_CUDA(adjoint_step<S>(h, st->seg[(size_t) (n - n0)], n));
+			ADJ_CUDA(adjoint_step<S>(h, n, moments_of(h, st->seg_mom, n - n0)));
 	}
 	return LBM_OK;
 }
@@ -240,13 +306,14 @@ int lbm_adjoint_forward(lbm_handle h, const double* force, int64_t nsteps, int64
 		if (g == lbm::GEO_INFLOW_LEFT || g == lbm::GEO_INFLOW_EQ_LEFT)
 			return afail(LBM_ERR_UNSUPPORTED, "the adjoint has no transpose of GEO_INFLOW_LEFT / GEO_INFLOW_EQ_LEFT; use GEO_INFLOW");
 	const long long nsites = h->sites();
-	std::set<long long> seen;
+	std::vector<bool> seen((size_t) nsites);
 	for (int i = 0; i < nsamples; i++) {
 		const long long s = samples[i];
 		if (s < 0 || s >= nsites)
 			return afail(LBM_ERR_INVALID, "sample %d: site index %lld out of range", i, s);
-		if (!seen.insert(s).second)
+		if (seen[(size_t) s])
 			return afail(LBM_ERR_INVALID, "sample %d: site %lld listed twice", i, s);
+		seen[(size_t) s] = true;
 		if (!h->d.periodic && h->map_host[(size_t) s] != lbm::GEO_FLUID && h->map_host[(size_t) s] != lbm::GEO_PERIODIC)
 			return afail(LBM_ERR_INVALID, "sample %d: site %lld is not a fluid site", i, s);
 	}
@@ -255,7 +322,7 @@ int lbm_adjoint_forward(lbm_handle h, const double* force, int64_t nsteps, int64
 		every = (long long) std::ceil(std::sqrt((double) nsteps));
 	if (every > nsteps)
 		every = nsteps;
-	const long long nckpt = (nsteps + every - 1) / every;
+	long long kept = kept_steps(h, nsteps, every);
 
 	// the buffers of an earlier run are kept and grown only when this run
 	// needs more (an optimisation loop reruns forward and backward)
@@ -301,6 +368,10 @@ int lbm_adjoint_forward(lbm_handle h, const double* force, int64_t nsteps, int64
 			return fail_free(afail(LBM_ERR_CUDA, "adjoint buffers: allocation failed"));
 		st->nsamples_cap = nsamples;
 	}
+	if (!ensure_bytes(st->kept_mom, st->kept_bytes, moments_bytes(h) * (size_t) kept))
+		kept = 0;  // no room: every step is recomputed
+	const long long nckpt = (nsteps - kept + every - 1) / every;
+	st->kept = kept;
 	while ((long long) st->ckpt.size() < nckpt) {
 		void* p = nullptr;
 		if (cudaMalloc(&p, h->pop_bytes) != cudaSuccess)
@@ -337,11 +408,12 @@ int lbm_adjoint_backward(lbm_handle h, double seed, double* grad_force, void* gr
 	const size_t pb = h->pop_bytes;
 	if (!st->lam && (cudaMalloc(&st->lam, lam_bytes(h)) != cudaSuccess || cudaMalloc(&st->grad, sizeof(double) * 3 * h->sites()) != cudaSuccess))
 		return afail(LBM_ERR_CUDA, "adjoint state allocation failed");
-	while ((long long) st->seg.size() < st->every) {
-		void* p = nullptr;
-		if (cudaMalloc(&p, pb) != cudaSuccess)
-			return afail(LBM_ERR_CUDA, "adjoint segment buffers: allocation of %lld x %zu bytes failed", st->every, pb);
-		st->seg.push_back(p);
+	if (st->nckpt > 0) {
+		if (!st->work && cudaMalloc(&st->work, pb) != cudaSuccess)
+			return afail(LBM_ERR_CUDA, "adjoint working array: allocation of %zu bytes failed", pb);
+		const size_t bytes = moments_bytes(h) * (size_t) st->every;
+		if (!ensure_bytes(st->seg_mom, st->seg_bytes, bytes))
+			return afail(LBM_ERR_CUDA, "adjoint segment moments: allocation of %zu bytes failed", bytes);
 	}
 	const int rc = h->ops->compute_size == 8 ? backward_typed<lbm::StoreF64>(h, seed) : backward_typed<lbm::StoreF32>(h, seed);
 	if (rc)
