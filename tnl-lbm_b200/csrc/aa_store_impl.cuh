@@ -174,12 +174,10 @@ struct StorageUnit
 		if (L.dry_run)
 			return cudaSuccess;
 		if (L.macro || L.partials)
-			aa_step_kernel<S, COLL, CUMF, ODD, GENERAL, true, direct_minb<R, COLL, CUMF, ODD, GENERAL, true>()>
-				<<<L.grid, L.block, 0, L.stream>>>(a);
-		else
-			aa_step_kernel<S, COLL, CUMF, ODD, GENERAL, false, direct_minb<R, COLL, CUMF, ODD, GENERAL, false>()>
-				<<<L.grid, L.block, 0, L.stream>>>(a);
-		return cudaGetLastError();
+			return launch_dependent(L.dependent, aa_step_kernel<S, COLL, CUMF, ODD, GENERAL, true, direct_minb<R, COLL, CUMF, ODD, GENERAL, true>()>,
+									L.grid, L.block, L.stream, a);
+		return launch_dependent(L.dependent, aa_step_kernel<S, COLL, CUMF, ODD, GENERAL, false, direct_minb<R, COLL, CUMF, ODD, GENERAL, false>()>,
+								L.grid, L.block, L.stream, a);
 	}
 
 	template <int COLL, int CUMF>
@@ -200,12 +198,10 @@ struct StorageUnit
 		if (L.dry_run)
 			return cudaSuccess;
 		if (L.macro || L.partials || d.phi)
-			ade_step_kernel<S, COLL, CUMF, ODD, GENERAL, true, ade_minb<R, COLL, CUMF, ODD, GENERAL, true>()>
-				<<<L.grid, L.block, 0, L.stream>>>(a, d);
-		else
-			ade_step_kernel<S, COLL, CUMF, ODD, GENERAL, false, ade_minb<R, COLL, CUMF, ODD, GENERAL, false>()>
-				<<<L.grid, L.block, 0, L.stream>>>(a, d);
-		return cudaGetLastError();
+			return launch_dependent(L.dependent, ade_step_kernel<S, COLL, CUMF, ODD, GENERAL, true, ade_minb<R, COLL, CUMF, ODD, GENERAL, true>()>,
+									L.grid, L.block, L.stream, a, d);
+		return launch_dependent(L.dependent, ade_step_kernel<S, COLL, CUMF, ODD, GENERAL, false, ade_minb<R, COLL, CUMF, ODD, GENERAL, false>()>,
+								L.grid, L.block, L.stream, a, d);
 	}
 
 	template <int COLL, int CUMF>
@@ -302,12 +298,10 @@ struct StorageUnit
 		if (L.dry_run)
 			return cudaSuccess;
 		if (L.macro || L.partials)
-			ab_step_kernel<S, COLL, CUMF, true, ab_minb<R, COLL, CUMF, true>()>
-				<<<L.grid, L.block, 0, L.stream>>>(a, (T*) L.f_out);
-		else
-			ab_step_kernel<S, COLL, CUMF, false, ab_minb<R, COLL, CUMF, false>()>
-				<<<L.grid, L.block, 0, L.stream>>>(a, (T*) L.f_out);
-		return cudaGetLastError();
+			return launch_dependent(L.dependent, ab_step_kernel<S, COLL, CUMF, true, ab_minb<R, COLL, CUMF, true>()>, L.grid, L.block, L.stream, a,
+									(T*) L.f_out);
+		return launch_dependent(L.dependent, ab_step_kernel<S, COLL, CUMF, false, ab_minb<R, COLL, CUMF, false>()>, L.grid, L.block, L.stream, a,
+								(T*) L.f_out);
 	}
 
 	static cudaError_t ab_step(const StepLaunch& L)

@@ -129,6 +129,8 @@ __global__ void __launch_bounds__(128, MINB)
 	ab_step_kernel(const StepArgs<typename S::T, typename S::R> a, typename S::T* __restrict__ fout)
 {
 	using R = typename S::R;
+	launch_dependents();
+	await_predecessor();
 	const int x = blockIdx.x * blockDim.x + threadIdx.x;
 	const int y = blockIdx.y * blockDim.y + threadIdx.y;
 	const int z = blockIdx.z;

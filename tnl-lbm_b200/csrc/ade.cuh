@@ -349,6 +349,8 @@ template <typename S, int COLL, int CUMF, bool ODD, bool GENERAL, bool OUT, int 
 __global__ void __launch_bounds__(128, MINB)
 	ade_step_kernel(const StepArgs<typename S::T, typename S::R> a, const AdeArgs<typename S::R> d)
 {
+	launch_dependents();
+	await_predecessor();
 	ade_site_update<S, COLL, CUMF, ODD, GENERAL, OUT>(a, d, blockIdx.x * blockDim.x + threadIdx.x,
 													  blockIdx.y * blockDim.y + threadIdx.y, blockIdx.z);
 }

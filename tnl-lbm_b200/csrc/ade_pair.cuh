@@ -118,6 +118,8 @@ __global__ void __launch_bounds__(128, MINB)
 						 const PairSlots psd, const PairRows pr, const AdeArgs<float> d, const uint8_t* __restrict__ groups,
 						 const unsigned* __restrict__ work, const unsigned long long* __restrict__ rest, long long nrest)
 {
+	launch_dependents();
+	await_predecessor();
 	const unsigned w = work[blockIdx.x];
 	if (w & PAIR_WORK_REST) {
 		const long long i = (long long) (w & ~PAIR_WORK_REST) * 128 + threadIdx.x;
@@ -135,7 +137,7 @@ __global__ void __launch_bounds__(128, MINB)
 	}
 	else {
 		int x, y, z;
-		const bool act = pair_position(pr, w * 128 + threadIdx.x, x, y, z);
+		const bool act = pair_position(pr, w, x, y, z);
 		ade_pair_update<S, CUMF, ODD>(a, p2, ps, psd, d, groups, act, x, y, z);
 	}
 }
@@ -211,14 +213,15 @@ cudaError_t ade_pair_step(const StepLaunch& L)
 	PairRows pr;
 	if (!make_pair_rows(L.g.X, L.g.Y, L.g.Z, pr))
 		return cudaErrorNotSupported;
+	cudaError_t err = cudaSuccess;
 #define LBM_ADE_PAIR(CUMF)                                                                                             \
 	do {                                                                                                               \
 		if (L.odd)                                                                                                     \
-			ade_pair_work_kernel<S, CUMF, true, ADE_PAIR_MINB_ODD>                                                         \
-				<<<grid, block, 0, L.stream>>>(a, p2, ps, psd, pr, d, A->pair_groups, W.work, W.rest, W.nrest);                 \
+			err = launch_dependent(L.dependent, ade_pair_work_kernel<S, CUMF, true, ADE_PAIR_MINB_ODD>, grid, block, L.stream, \
+								   a, p2, ps, psd, pr, d, A->pair_groups, W.work, W.rest, W.nrest);                       \
 		else                                                                                                           \
-			ade_pair_work_kernel<S, CUMF, false, ADE_PAIR_MINB_EVEN>                                                        \
-				<<<grid, block, 0, L.stream>>>(a, p2, ps, psd, pr, d, A->pair_groups, W.work, W.rest, W.nrest);                 \
+			err = launch_dependent(L.dependent, ade_pair_work_kernel<S, CUMF, false, ADE_PAIR_MINB_EVEN>, grid, block, L.stream, \
+								   a, p2, ps, psd, pr, d, A->pair_groups, W.work, W.rest, W.nrest);                        \
 	} while (0)
 	switch (L.cum_flags) {
 		case 0:
@@ -232,7 +235,7 @@ cudaError_t ade_pair_step(const StepLaunch& L)
 			break;
 	}
 #undef LBM_ADE_PAIR
-	return cudaGetLastError();
+	return err;
 }
 
 }  // namespace lbm

@@ -37,37 +37,42 @@ inline Geometry make_geometry(int X, int Y, int Z, int es, int slots = 27)
 	return g;
 }
 
-// Work list of the two-site kernels on a lattice with a map (pair.cuh): per z
-// plane the chunks of 128 rest sites that start in it (rest[i] = row << 32 | x),
-// then the tiles of 128 pairs (linear order, ceil(X / 2) pairs to a row) that
-// start in it and hold a pair group.  The slower per-site work starts first
-// and the tiles fill in around it (duct 26.7 -> 28.3 GLUPS against chunks
-// after the tiles).  false: more items than the list numbers.
-inline bool build_pair_work(int X, int Y, int Z, const std::vector<uint8_t>& groups,
-							const std::vector<unsigned long long>& rest, std::vector<unsigned>& work)
+// The tiles of 128 pairs that hold a pair group: those its first and last pair
+// lie in (the PAIR_GROUP / 2 pairs of a group reach into two tiles at most).
+inline std::vector<uint8_t> pair_tiles(int X, int Y, int Z, const std::vector<uint8_t>& groups)
 {
-	const long long px = X / 2 + X % 2, npairs = px * Y * Z;
-	const long long gx = (X + PAIR_GROUP - 1) / PAIR_GROUP;
-	const long long nchunks = ((long long) rest.size() + 127) / 128;
-	if (nchunks >= (long long) PAIR_WORK_REST - 1 || npairs >= (1ll << 31) - 1024)
-		return false;
-	// tiles that hold a pair group: those its first and last pair lie in (a
-	// group's PAIR_GROUP / 2 pairs reach into two tiles at most)
-	std::vector<bool> any((size_t) ((npairs + 127) / 128));
+	const long long px = X / 2 + X % 2, gx = (X + PAIR_GROUP - 1) / PAIR_GROUP;
+	std::vector<uint8_t> tiles((size_t) ((px * Y * Z + 127) / 128));
 	const uint8_t* g = groups.data();
 	for (long long row = 0; row < (long long) Y * Z; row++)
 		for (long long k = 0; k < gx; k++, g++)
 			if (*g != PAIR_GROUP_REST) {
 				const long long first = row * px + k * (PAIR_GROUP / 2);
-				any[(size_t) (first / 128)] = true;
-				any[(size_t) ((first + PAIR_GROUP / 2 - 1) / 128)] = true;
+				tiles[(size_t) (first / 128)] = 1;
+				tiles[(size_t) ((first + PAIR_GROUP / 2 - 1) / 128)] = 1;
 			}
+	return tiles;
+}
+
+// Work list of the two-site kernels on a lattice with a map (pair.cuh): per z
+// plane the chunks of 128 rest sites that start in it (rest[i] = row << 32 | x),
+// then the tiles of 128 pairs (linear order, ceil(X / 2) pairs to a row) that
+// start in it and hold a pair group (pair_tiles).  The slower per-site work starts first
+// and the tiles fill in around it (duct 26.7 -> 28.3 GLUPS against chunks
+// after the tiles).  false: more items than the list numbers.
+inline bool build_pair_work(int X, int Y, int Z, const std::vector<uint8_t>& tiles,
+							const std::vector<unsigned long long>& rest, std::vector<unsigned>& work)
+{
+	const long long px = X / 2 + X % 2;
+	const long long nchunks = ((long long) rest.size() + 127) / 128, ntiles = (long long) tiles.size();
+	if (nchunks >= (long long) PAIR_WORK_REST - 1 || px * Y * Z >= (1ll << 31) - 1024)
+		return false;
 	long long c = 0, t = 0;
 	for (int z = 0; z < Z; z++) {
 		while (c < nchunks && (long long) (rest[(size_t) c * 128] >> 32) / Y <= z)
 			work.push_back(PAIR_WORK_REST | (unsigned) c++);
-		for (; t < (long long) any.size() && t * 128 < (z + 1) * px * Y; t++)
-			if (any[(size_t) t])
+		for (; t < ntiles && t * 128 < (z + 1) * px * Y; t++)
+			if (tiles[(size_t) t])
 				work.push_back((unsigned) t);
 	}
 	return true;

@@ -9,6 +9,29 @@
 
 namespace lbm {
 
+// Launches a step kernel as a programmatic dependent of the kernel before it on
+// the stream: its blocks are scheduled while that kernel's last ones run and
+// wait in await_predecessor (aa_kernels.cuh).  After anything but a kernel (a
+// copy, a wait on an event) it starts as an ordinary launch.  Only for kernels
+// whose every thread begins with await_predecessor: one that did not wait could
+// complete, and let its own dependents go, ahead of its predecessor.
+// dependent = false: an ordinary launch.
+template <typename... P, typename... A>
+inline cudaError_t launch_dependent(bool dependent, void (*kernel)(P...), dim3 grid, dim3 block, cudaStream_t stream, A... args)
+{
+	cudaLaunchAttribute attr;
+	attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+	attr.val.programmaticStreamSerializationAllowed = 1;
+	cudaLaunchConfig_t cfg = {};
+	cfg.gridDim = grid;
+	cfg.blockDim = block;
+	cfg.stream = stream;
+	cfg.attrs = &attr;
+	cfg.numAttrs = dependent ? 1 : 0;
+	return cudaLaunchKernelEx(&cfg, kernel, P(args)...);
+}
+
+
 enum Storage : int
 {
 	ST_F64 = 0,
@@ -92,6 +115,9 @@ struct StepLaunch
 	// set by a step whose partial sums leave out the GEO_NOTHING sites (a
 	// sums-only step of the pair kernel over the plain work list), or null
 	bool* nothing_skipped;
+	// the launch may be a programmatic dependent of the kernel before it on the
+	// stream (launch_dependent): a lattice's own steps, one after the other
+	bool dependent;
 };
 
 // the coupled D3Q7 advection-diffusion scalar of a lattice (ade.cuh)

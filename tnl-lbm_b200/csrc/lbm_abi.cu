@@ -233,6 +233,7 @@ int launch_step(lbm_handle h, bool macro, bool sums, bool dry_run = false)
 	L.pair_work = lbm::PairWork{h->pair_work[0], h->pair_nwork[0], h->pair_rest[0], h->pair_nrest[0]};
 	L.pair_work_out = lbm::PairWork{h->pair_work[1], h->pair_nwork[1], h->pair_rest[1], h->pair_nrest[1]};
 	L.distributed_z = h->distributed_z;
+	L.dependent = true;
 	const bool ab = h->streaming == LBM_STREAMING_AB;
 	if (h->ade) {
 		h->ade->launch.phi = macro ? h->ade->phi_buf : nullptr;
@@ -638,8 +639,9 @@ int lbm_set_map(lbm_handle h, const uint8_t* map)
 					}
 			}
 		std::vector<unsigned> work[2];
+		const std::vector<uint8_t> tiles = lbm::pair_tiles(X, Y, Z, groups);
 		for (int k = 0; k < 2; k++)
-			if (!lbm::build_pair_work(X, Y, Z, groups, rest[k], work[k]))
+			if (!lbm::build_pair_work(X, Y, Z, tiles, rest[k], work[k]))
 				return fail(LBM_ERR_SIZE, "lattice too large for the pair step's work list");
 		cudaFree(h->pair_groups);
 		h->pair_groups = nullptr;

@@ -78,7 +78,7 @@ int ade_build_pair(lbm_lattice* h)
 						rest.push_back((unsigned long long) row << 32 | (unsigned) x);
 		}
 	std::vector<unsigned> work;
-	if (!build_pair_work(X, Y, Z, groups, rest, work))
+	if (!build_pair_work(X, Y, Z, pair_tiles(X, Y, Z, groups), rest, work))
 		return 0;
 	if (work.empty())
 		return 0;

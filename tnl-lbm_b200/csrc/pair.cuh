@@ -526,9 +526,11 @@ inline bool make_pair_rows(int X, int Y, int Z, PairRows& pr)
 	return true;
 }
 
-// first site (x, y, z) of pair p; false past the last pair
-__device__ __forceinline__ bool pair_position(const PairRows& pr, unsigned p, int& x, int& y, int& z)
+// first site (x, y, z) of the thread's pair in block `item` of the linear
+// order; false past the last pair
+__device__ __forceinline__ bool pair_position(const PairRows& pr, unsigned item, int& x, int& y, int& z)
 {
+	const unsigned p = item * blockDim.x + threadIdx.x;
 	const unsigned row = fast_div(p, pr.px);
 	x = 2 * (int) (p - row * (unsigned) pr.px.d);
 	z = (int) fast_div(row, pr.y);
@@ -689,11 +691,11 @@ template <typename S, typename C, bool ODD, bool OUT, bool RAGGED, int MINB>
 __global__ void __launch_bounds__(128, MINB) aa_pair_kernel(const StepArgs<typename S::T, float> a, const CollParams<F2> p2,
 															 const PairSlots ps, const PairRows pr, long long red_slots)
 {
-	if constexpr (OUT)
-		launch_dependents();
+	launch_dependents();
+	await_predecessor();
 	const long long slot = (long long) blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
 	int x, y, z;
-	const bool act = pair_position(pr, blockIdx.x * blockDim.x + threadIdx.x, x, y, z);
+	const bool act = pair_position(pr, blockIdx.x, x, y, z);
 	pair_update<S, C, ODD, false, OUT, RAGGED>(a, p2, ps, nullptr, act, x, y, z, slot, red_slots);
 }
 
@@ -710,8 +712,8 @@ __global__ void __launch_bounds__(128, MINB)
 						const uint8_t* __restrict__ groups, const unsigned* __restrict__ work,
 						const unsigned long long* __restrict__ rest, long long nrest)
 {
-	if constexpr (OUT)
-		launch_dependents();
+	launch_dependents();
+	await_predecessor();
 	const unsigned w = work[blockIdx.x];
 	const long long slot = (long long) blockIdx.x * 4 + (threadIdx.x >> 5);
 	const long long nslots = (long long) gridDim.x * 4;
@@ -720,7 +722,7 @@ __global__ void __launch_bounds__(128, MINB)
 	}
 	else {
 		int x, y, z;
-		const bool act = pair_position(pr, w * 128 + threadIdx.x, x, y, z);
+		const bool act = pair_position(pr, w, x, y, z);
 		pair_update<S, C, ODD, true, OUT, false>(a, p2, ps, groups, act, x, y, z, slot, nslots);
 	}
 }
@@ -774,6 +776,7 @@ cudaError_t pair_step_with(const StepLaunch& L)
 	// GEO_NOTHING sites (they output rho = 1, u = 0); a sums-only step runs
 	// the plain list, and the finish kernel adds those sites' rho = 1 each
 	const PairWork& W = L.macro ? L.pair_work_out : L.pair_work;
+	const unsigned threads = general ? 128 : L.block.x * L.block.y;
 	PairRows pr;
 	if ((general && (!W.work || !L.pair_groups || W.nwork < 1)) || !make_pair_rows(L.g.X, L.g.Y, L.g.Z, pr))
 		return cudaErrorNotSupported;
@@ -802,7 +805,6 @@ cudaError_t pair_step_with(const StepLaunch& L)
 	if (27ll * L.g.sq * (long long) sizeof(T) >= (1ll << 31))
 		return cudaErrorNotSupported;
 	const PairSlots ps = make_pair_slots(L.g.sq, (int) sizeof(T));
-	const unsigned threads = general ? 128 : L.block.x * L.block.y;
 	const unsigned grid = general ? (unsigned) W.nwork : (pr.npairs + threads - 1) / threads;
 	// one partial-sum slot per warp
 	const long long red_slots = (long long) grid * (threads / 32);
@@ -813,34 +815,36 @@ cudaError_t pair_step_with(const StepLaunch& L)
 	if (L.dry_run)
 		return cudaSuccess;
 	const bool ragged = L.g.X % 2 != 0;
+	cudaError_t err = cudaSuccess;
 	auto launch = [&](auto odd)
 	{
 		constexpr bool ODD = decltype(odd)::value;
 		constexpr int MINB = C::template pair_minb<T, ODD>();
 		if (general) {
+			auto go = [&](auto kern)
+			{ err = launch_dependent(L.dependent, kern, grid, threads, L.stream, a, p2, ps, pr, L.pair_groups, W.work, W.rest, W.nrest); };
 			if (out)
-				aa_pair_work_kernel<S, C, ODD, true, MINB>
-					<<<grid, threads, 0, L.stream>>>(a, p2, ps, pr, L.pair_groups, W.work, W.rest, W.nrest);
+				go(aa_pair_work_kernel<S, C, ODD, true, MINB>);
 			else
-				aa_pair_work_kernel<S, C, ODD, false, MINB>
-					<<<grid, threads, 0, L.stream>>>(a, p2, ps, pr, L.pair_groups, W.work, W.rest, W.nrest);
+				go(aa_pair_work_kernel<S, C, ODD, false, MINB>);
 		}
-		else if (ragged) {
-			if (out)
-				aa_pair_kernel<S, C, ODD, true, true, MINB><<<grid, threads, 0, L.stream>>>(a, p2, ps, pr, red_slots);
+		else {
+			auto go = [&](auto kern) { err = launch_dependent(L.dependent, kern, grid, threads, L.stream, a, p2, ps, pr, red_slots); };
+			if (ragged && out)
+				go(aa_pair_kernel<S, C, ODD, true, true, MINB>);
+			else if (ragged)
+				go(aa_pair_kernel<S, C, ODD, false, true, MINB>);
+			else if (out)
+				go(aa_pair_kernel<S, C, ODD, true, false, MINB>);
 			else
-				aa_pair_kernel<S, C, ODD, false, true, MINB><<<grid, threads, 0, L.stream>>>(a, p2, ps, pr, red_slots);
+				go(aa_pair_kernel<S, C, ODD, false, false, MINB>);
 		}
-		else if (out)
-			aa_pair_kernel<S, C, ODD, true, false, MINB><<<grid, threads, 0, L.stream>>>(a, p2, ps, pr, red_slots);
-		else
-			aa_pair_kernel<S, C, ODD, false, false, MINB><<<grid, threads, 0, L.stream>>>(a, p2, ps, pr, red_slots);
 	};
 	if (L.odd)
 		launch(std::true_type{});
 	else
 		launch(std::false_type{});
-	return cudaGetLastError();
+	return err;
 }
 
 // One A-A step of the lattice's built-in collision on the two-site kernels;

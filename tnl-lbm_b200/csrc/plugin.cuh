@@ -68,8 +68,8 @@ __global__ void __launch_bounds__(128, plugin_minb<typename S::R>())
 	aa_step_plugin_kernel(const StepArgs<typename S::T, typename S::R> a)
 {
 	using R = typename S::R;
-	if constexpr (OUT)
-		launch_dependents();
+	launch_dependents();
+	await_predecessor();
 	aa_step_site<S, ODD, GENERAL, OUT>(a, [&](Site<R>& s) { C::template collision<R>(s, a.p); });
 }
 
@@ -95,10 +95,8 @@ cudaError_t plugin_launch(const StepLaunch& L)
 {
 	const StepArgs<typename S::T, typename S::R> a = make_step_args<S>(L);
 	if (L.macro || L.partials)
-		aa_step_plugin_kernel<S, C, ODD, GENERAL, true><<<L.grid, L.block, 0, L.stream>>>(a);
-	else
-		aa_step_plugin_kernel<S, C, ODD, GENERAL, false><<<L.grid, L.block, 0, L.stream>>>(a);
-	return cudaGetLastError();
+		return launch_dependent(L.dependent, aa_step_plugin_kernel<S, C, ODD, GENERAL, true>, L.grid, L.block, L.stream, a);
+	return launch_dependent(L.dependent, aa_step_plugin_kernel<S, C, ODD, GENERAL, false>, L.grid, L.block, L.stream, a);
 }
 
 // one step of storage S: the launch shape and the partial-sum slots of the
