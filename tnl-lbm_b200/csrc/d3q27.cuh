@@ -213,11 +213,22 @@ struct StoreF16S
 {
 	using T = __half;
 	using R = float;
+	// h / s + w as one mixed-precision multiply-add of sm_100 (half operands, float
+	// sum): the product by a power of two is exact, so the value is that of a
+	// conversion and a float multiply-add, in one instruction for both
+	template <int Q>
+	__device__ static __forceinline__ R from_raw(unsigned short raw)
+	{
+		// the half 1 / s = 2^-k: exponent field 15 - k, mantissa 0
+		constexpr int k = half_scale(Q) == 4.0f ? 2 : half_scale(Q) == 16.0f ? 4 : half_scale(Q) == 64.0f ? 6 : 8;
+		R v;
+		asm("fma.rn.f32.f16 %0, %1, %2, %3;" : "=f"(v) : "h"(raw), "h"((unsigned short) ((15 - k) << 10)), "f"((float) weight(Q)));
+		return v;
+	}
 	template <int Q>
 	__device__ static __forceinline__ R load(const T* p)
 	{
-		const unsigned short raw = __ldcs(reinterpret_cast<const unsigned short*>(p));
-		return __half2float(__ushort_as_half(raw)) * (1.0f / half_scale(Q)) + (float) weight(Q);
+		return from_raw<Q>(__ldcs(reinterpret_cast<const unsigned short*>(p)));
 	}
 	// (v - w) * s as one fused multiply-add, v * s - w * s with w * s exact
 	// (s a power of two): one rounding instead of two, one instruction less
@@ -235,7 +246,7 @@ struct StoreF16S
 	template <int Q>
 	__device__ static __forceinline__ R load_smem(const T* p)
 	{
-		return __half2float(*p) * (1.0f / half_scale(Q)) + (float) weight(Q);
+		return from_raw<Q>(__half_as_ushort(*p));
 	}
 };
 
@@ -272,11 +283,18 @@ struct StoreBF16S
 {
 	using T = __nv_bfloat16;
 	using R = float;
+	// as StoreF16S: the conversion and the addition of w in one instruction
+	template <int Q>
+	__device__ static __forceinline__ R from_raw(unsigned short raw)
+	{
+		R v;
+		asm("add.rn.f32.bf16 %0, %1, %2;" : "=f"(v) : "h"(raw), "f"((float) weight(Q)));
+		return v;
+	}
 	template <int Q>
 	__device__ static __forceinline__ R load(const T* p)
 	{
-		const unsigned short raw = __ldcs(reinterpret_cast<const unsigned short*>(p));
-		return __bfloat162float(__ushort_as_bfloat16(raw)) + (float) weight(Q);
+		return from_raw<Q>(__ldcs(reinterpret_cast<const unsigned short*>(p)));
 	}
 	template <int Q>
 	__device__ static __forceinline__ void store(T* p, R v)
@@ -287,7 +305,7 @@ struct StoreBF16S
 	template <int Q>
 	__device__ static __forceinline__ R load_smem(const T* p)
 	{
-		return __bfloat162float(*p) + (float) weight(Q);
+		return from_raw<Q>(__bfloat16_as_ushort(*p));
 	}
 };
 

@@ -163,8 +163,8 @@ struct PairIO<StoreF16S>
 	template <int Q>
 	__device__ static __forceinline__ F2 load2(const __half* p)
 	{
-		const F2 h(__half22float2(__ldcs(reinterpret_cast<const __half2*>(p))));
-		return fma2(h, F2(1.0 / half_scale(Q)), F2(weight(Q)));
+		const unsigned w = __ldcs(reinterpret_cast<const unsigned*>(p));
+		return F2(StoreF16S::from_raw<Q>((unsigned short) w), StoreF16S::from_raw<Q>((unsigned short) (w >> 16)));
 	}
 	// (v - w) * s as v * s - w * s, as StoreF16S::scaled_deviation
 	template <int Q>
@@ -198,7 +198,8 @@ struct PairIO<StoreBF16S>
 	template <int Q>
 	__device__ static __forceinline__ F2 load2(const __nv_bfloat16* p)
 	{
-		return F2(__bfloat1622float2(__ldcs(reinterpret_cast<const __nv_bfloat162*>(p)))) + F2(weight(Q));
+		const unsigned w = __ldcs(reinterpret_cast<const unsigned*>(p));
+		return F2(StoreBF16S::from_raw<Q>((unsigned short) w), StoreBF16S::from_raw<Q>((unsigned short) (w >> 16)));
 	}
 	template <int Q>
 	__device__ static __forceinline__ void store2(__nv_bfloat16* p, F2 v)
@@ -572,19 +573,40 @@ __device__ __forceinline__ void pair_update(const StepArgs<typename S::T, float>
 		site = ((long long) z * a.Y + y) * a.X + x;
 		if constexpr (GENERAL) {
 			// a pair away from every lattice face has the same neighbours
-			// whether it wraps or not: its loads are issued together with the
-			// group flag's (and are discarded if the group is not a pair group)
+			// whether it wraps or not: its loads do not wait for the group flag
+			// (and are discarded if the group is not a pair group).  At the faces
+			// the flag comes first.
 			const bool inner = x > 0 && x + 2 < a.X && y > 0 && y < a.Y - 1 && z > 0 && z < a.Z - 1;
-			if (inner) {
-				at = pair_at(a, x, y, z, false);
-				pair_read_at<S, ODD>(at, ps, s);
-			}
 			const int gx = (a.X + PAIR_GROUP - 1) / PAIR_GROUP;
-			const uint8_t g = groups[((long long) z * a.Y + y) * gx + x / PAIR_GROUP];
-			act = g != PAIR_GROUP_REST;
-			if (act && !inner) {
-				at = pair_at(a, x, y, z, g == PAIR_GROUP_PERIODIC);
-				pair_read_at<S, ODD>(at, ps, s);
+			const uint8_t* const flag = groups + ((long long) z * a.Y + y) * gx + x / PAIR_GROUP;
+			if constexpr (sizeof(typename S::T) == 2) {
+				// one copy of the loads for both kinds, behind two predicated
+				// reads of the flag: the odd step spills 8 bytes instead of 60 and
+				// the even one 4 instead of 20.  (With 32-bit storage this form
+				// needs the warp sync below, which costs SRT 3 %.)
+				uint8_t at_face = PAIR_GROUP_FLUID, inside = PAIR_GROUP_FLUID;
+				if (inner)
+					inside = *flag;
+				else
+					at_face = *flag;
+				act = at_face != PAIR_GROUP_REST;
+				if (act) {
+					at = pair_at(a, x, y, z, at_face == PAIR_GROUP_PERIODIC);
+					pair_read_at<S, ODD>(at, ps, s);
+					act = inside != PAIR_GROUP_REST;
+				}
+			}
+			else {
+				if (inner) {
+					at = pair_at(a, x, y, z, false);
+					pair_read_at<S, ODD>(at, ps, s);
+				}
+				const uint8_t g = *flag;
+				act = g != PAIR_GROUP_REST;
+				if (act && !inner) {
+					at = pair_at(a, x, y, z, g == PAIR_GROUP_PERIODIC);
+					pair_read_at<S, ODD>(at, ps, s);
+				}
 			}
 		}
 		else {
