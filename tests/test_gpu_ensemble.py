@@ -126,6 +126,28 @@ def test_autotune_restores_state_and_picks_a_shape(pl):
     ens.close()
 
 
+@pytest.mark.parametrize("shape", [(128, 0), (128, 1), (256, 1), (256, 3)])
+def test_groups_of_members(pl, shape):
+    """An ensemble larger than one L2 group (several of 64 MB, one member larger
+    than a group, tiny members between them) runs group by group: members of
+    every group against single lattices, over an odd start, graph replays and a
+    remainder, and the sums of all members in one launch."""
+    sizes = [(64, 32, 32)] * 9 + [(96, 96, 96), (8, 4, 4)] + [(48, 40, 36)] * 10 + [(8, 6, 4), (64, 48, 32)]
+    nus = list(np.linspace(0.002, 0.03, len(sizes)))
+    ens = pl.Ensemble(sizes, nus, cum_flags=3, storage=pl.STORE_F32)
+    ens.set_shape(*shape)
+    ens.init_taylor_green(0.05)
+    ens.step(21)
+    ens.step(22, sums=True)
+    sums = ens.sums()
+    assert ens.iteration == 43
+    for m in (0, 8, 9, 10, 11, 20, 21, 22):
+        f_single, s_single = single_run(pl, sizes[m], nus[m], pl.STORE_F32, pl.COLL_CUM, 3, pl.EQ_INV_CUM, 43)
+        assert rel_linf(ens.get_populations(m), f_single) <= TOL["F32"], f"member {m}"
+        np.testing.assert_allclose(sums[m, :5], s_single[:5], rtol=1e-6, atol=1e-6 * abs(s_single[0]))
+    ens.close()
+
+
 def test_invalid_ensembles_are_rejected(pl):
     with pytest.raises(pl.LbmError) as e:
         pl.Ensemble([(8, 8, 8), (0, 4, 4)], [0.01, 0.01])

@@ -379,16 +379,16 @@ struct StorageUnit
 			sms_cache[dev] = sms;
 		}
 		long long grid = L.grid > 0 ? L.grid : (long long) per_sm_cache[dev] * sms_cache[dev];
-		if (grid > L.ntiles)
-			grid = L.ntiles;
+		if (grid > L.tile_end - L.tile_begin)
+			grid = L.tile_end - L.tile_begin;
 		if (grid > 0x7fffffffLL)
 			grid = 0x7fffffffLL;
 		if (L.blocks_out)
 			*L.blocks_out = grid;
 		if (L.dry_run || grid < 1)
 			return cudaSuccess;
-		kern<<<(unsigned) grid, TPB, 0, L.stream>>>((const EnsMember<T, R>*) L.members, L.tile_member, L.ntiles, L.partials);
-		return cudaGetLastError();
+		return launch_dependent(true, kern, (unsigned) grid, TPB, L.stream, (const EnsMember<T, R>*) L.members, L.tile_member,
+								L.ntiles, L.tile_begin, L.tile_end, L.partials);
 	}
 
 	// grid policy 3: the persistent two-site kernel over tiles of 256 sites
@@ -421,15 +421,14 @@ struct StorageUnit
 				sms_cache[dev] = sms;
 			}
 			long long grid = (long long) per_sm_cache[dev] * sms_cache[dev];
-			if (grid > L.ntiles)
-				grid = L.ntiles;
+			if (grid > L.tile_end - L.tile_begin)
+				grid = L.tile_end - L.tile_begin;
 			if (L.blocks_out)
 				*L.blocks_out = grid;
 			if (L.dry_run || grid < 1)
 				return cudaSuccess;
-			kern<<<(unsigned) grid, 128, 0, L.stream>>>((const EnsMember<T, float>*) L.members, L.tile_member, L.ntiles,
-														L.partials);
-			return cudaGetLastError();
+			return launch_dependent(true, kern, (unsigned) grid, 128, L.stream, (const EnsMember<T, float>*) L.members,
+									L.tile_member, L.ntiles, L.tile_begin, L.tile_end, L.partials);
 		}
 	}
 

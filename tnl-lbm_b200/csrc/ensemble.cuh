@@ -37,12 +37,12 @@ struct EnsMember
 	CollParams<F2> p2;	// the same constants in both lanes (two-site kernel)
 };
 
-// One A-A step of every member.  OUT: per-tile FP64 partial sums
+// One A-A step of the members of tiles [tile_begin, tile_end).  OUT: per-tile FP64 partial sums
 // (partials[k * ntiles + tile]) of the sums of lbm_get_sums.
 template <typename S, int COLL, int CUMF, bool ODD, bool OUT, int TPB, int MINB>
 __global__ void __launch_bounds__(TPB, MINB)
 	ens_step_kernel(const EnsMember<typename S::T, typename S::R>* __restrict__ members, const int* __restrict__ tile_member,
-					long long ntiles, double* __restrict__ partials)
+					long long ntiles, long long tile_begin, long long tile_end, double* __restrict__ partials)
 {
 	using T = typename S::T;
 	using R = typename S::R;
@@ -51,8 +51,10 @@ __global__ void __launch_bounds__(TPB, MINB)
 	__shared__ EnsMember<T, R> M;
 	constexpr int WORDS = (int) (sizeof(EnsMember<T, R>) / 4);
 	static_assert(sizeof(EnsMember<T, R>) % 4 == 0 && WORDS <= TPB, "member entry size");
+	launch_dependents();
+	await_predecessor();
 	int cur = -1;
-	for (long long t = blockIdx.x; t < ntiles; t += gridDim.x) {
+	for (long long t = tile_begin + blockIdx.x; t < tile_end; t += gridDim.x) {
 		const int m = tile_member[t];
 		if (m != cur) {
 			__syncthreads();  // every thread is done with the previous entry
@@ -114,7 +116,7 @@ __global__ void __launch_bounds__(TPB, MINB)
 	}
 }
 
-// One A-A step of every member, two x-adjacent sites per thread (grid policy
+// The same, two x-adjacent sites per thread (grid policy
 // 3): tiles of 256 sites, 128 threads, the per-pair code of aa_pair_kernel
 // with the member's constants.  The grid walks the tile list with a stride
 // of the grid size, so the blocks resident at one time work on neighbouring
@@ -125,7 +127,7 @@ __global__ void __launch_bounds__(TPB, MINB)
 template <typename S, int COLL, int CUMF, bool ODD, bool OUT, int MINB>
 __global__ void __launch_bounds__(128, MINB)
 	ens_pair_kernel(const EnsMember<typename S::T, float>* __restrict__ members, const int* __restrict__ tile_member,
-					long long ntiles, double* __restrict__ partials)
+					long long ntiles, long long tile_begin, long long tile_end, double* __restrict__ partials)
 {
 	using T = typename S::T;
 	__shared__ EnsMember<T, float> M;
@@ -134,8 +136,10 @@ __global__ void __launch_bounds__(128, MINB)
 	__shared__ PairSlots ps;
 	constexpr int WORDS = (int) (sizeof(EnsMember<T, float>) / 4);
 	static_assert(sizeof(EnsMember<T, float>) % 4 == 0 && WORDS <= 128, "member entry size");
+	launch_dependents();
+	await_predecessor();
 	int cur = -1;
-	for (long long t = blockIdx.x; t < ntiles; t += gridDim.x) {
+	for (long long t = tile_begin + blockIdx.x; t < tile_end; t += gridDim.x) {
 		const int m = tile_member[t];
 		if (m != cur) {
 			__syncthreads();

@@ -169,7 +169,8 @@ struct EnsLaunch
 {
 	const void* members;	 // device table of the storage's EnsMember entries
 	const int* tile_member;	 // member of each tile
-	long long ntiles;
+	long long ntiles;		 // of the ensemble
+	long long tile_begin, tile_end;	 // tiles this launch updates
 	int tpb;		   // sites per tile = threads per block: 128 or 256
 	bool pair;		   // two sites per thread (tpb = 256 sites on 128 threads, cumulant, FP32 arithmetic)
 	long long grid;	   // blocks; 0 = resident blocks per SM x SMs (persistent)

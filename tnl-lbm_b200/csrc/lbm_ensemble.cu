@@ -93,6 +93,7 @@ struct lbm_ensemble_t
 	int grid_policy = 0;
 	long long ntiles = 0;
 	std::vector<long long> tile0;  // [count + 1]
+	std::vector<int> group0;	   // first member of each group of members that runs its steps together, and count
 	void* members_dev = nullptr;
 	int* tile_member_dev = nullptr;
 	long long* tile0_dev = nullptr;
@@ -201,10 +202,48 @@ int ensure_lanes(lbm_ensemble e)
 	return LBM_OK;
 }
 
+// Members are independent of one another, so a block of steps runs group by
+// group: the populations of a group of small members stay in L2 from step to
+// step instead of passing through HBM once per step.  Members in order, a group
+// closed when the next member would take it past ENS_GROUP_BYTES (a member
+// larger than that is a group of its own, which costs it nothing) unless it
+// would leave a group too small to fill the GPU.  B200 (126 MB of L2), us a step
+// for groups of 24, 32, 48, 64, 96 MB and one group: 128 members of 16-32 sites a
+// side 88, 85, 81, 79, 89, 89 (one site per thread); 512 of 16-32 319, 345, 294,
+// 288, 366, 383 and 64 of 32-128 1069, 1066, 1056, 1062, 1093, 1163 (two sites).
+#ifndef ENS_GROUP_BYTES
+#define ENS_GROUP_BYTES (64ll << 20)
+#endif
+void build_groups(lbm_ensemble e)
+{
+	e->group0.assign(1, 0);
+	long long total = 0;
+	std::vector<long long> bytes(e->count);
+	for (int m = 0; m < e->count; m++) {
+		const lbm::Geometry& g = e->g[m];
+		// the lines a step touches: 27 rows of X elements in 128-byte lines
+		const long long line = ((long long) g.X * e->ops->elem_size + 127) / 128 * 128;
+		bytes[m] = 27 * line * g.Y * g.Z;
+		total += bytes[m];
+	}
+	// equal shares of the whole
+	const long long n = (total + ENS_GROUP_BYTES - 1) / ENS_GROUP_BYTES;
+	const long long share = (total + n - 1) / n;
+	long long acc = 0;
+	for (int m = 0; m < e->count; m++) {
+		if (acc > share / 2 && acc + bytes[m] / 2 > share) {
+			e->group0.push_back(m);
+			acc = 0;
+		}
+		acc += bytes[m];
+	}
+	e->group0.push_back(e->count);
+}
+
 // grid policy 2: every member runs the single-lattice step (the two-site
 // kernel where it applies, else the direct kernel) on its lane; the lanes fork from and join into the ensemble's stream, so under
 // graph capture the members become independent branches
-int ens_launch_members(lbm_ensemble e)
+int ens_launch_members(lbm_ensemble e, long long iteration)
 {
 	if (int rc = ensure_lanes(e))
 		return rc;
@@ -219,7 +258,7 @@ int ens_launch_members(lbm_ensemble e)
 		L.p = e->p[m];
 		L.coll = e->collision;
 		L.cum_flags = e->cum_flags;
-		L.odd = (e->iteration % 2) != 0;
+		L.odd = (iteration % 2) != 0;
 		const int bx = g.X >= 128 ? 128 : ((g.X + 31) / 32) * 32;
 		L.block = dim3(bx, 128 / bx, 1);
 		L.grid = dim3((g.X + bx - 1) / bx, (g.Y + L.block.y - 1) / L.block.y, g.Z);
@@ -241,57 +280,60 @@ int ens_launch_members(lbm_ensemble e)
 	return LBM_OK;
 }
 
-int ens_launch(lbm_ensemble e, bool sums, bool dry_run = false)
+// one step of members [m0, m1) at the parity of `iteration` (grid policy 2: of all)
+int ens_launch(lbm_ensemble e, int m0, int m1, long long iteration, bool sums, bool dry_run = false)
 {
-	if (e->grid_policy == 2 && !sums) {
-		if (dry_run)
-			return LBM_OK;
-		if (int rc = ens_launch_members(e))
-			return rc;
-		e->iteration++;
-		return LBM_OK;
-	}
+	if (e->grid_policy == 2 && !sums)
+		return dry_run ? LBM_OK : ens_launch_members(e, iteration);
 	lbm::EnsLaunch L{};
 	L.members = e->members_dev;
 	L.tile_member = e->tile_member_dev;
 	L.ntiles = e->ntiles;
+	L.tile_begin = e->tile0[m0];
+	L.tile_end = e->tile0[m1];
 	L.tpb = e->tile_sites;
 	L.pair = e->grid_policy == 3;
-	L.grid = e->grid_policy == 1 ? e->ntiles : 0;
+	L.grid = e->grid_policy == 1 ? L.tile_end - L.tile_begin : 0;
 	L.partials = sums ? e->partials : nullptr;
 	L.coll = e->collision;
 	L.cum_flags = e->cum_flags;
-	L.odd = (e->iteration % 2) != 0;
+	L.odd = (iteration % 2) != 0;
 	L.stream = e->stream;
 	L.dry_run = dry_run;
 	const cudaError_t err = e->ops->ens_step(L);
 	if (err != cudaSuccess)
 		return efail(LBM_ERR_CUDA, "ensemble step launch failed: %s", cudaGetErrorString(err));
-	if (!dry_run)
-		e->iteration++;
+	return LBM_OK;
+}
+
+// n steps of every member from the parity of `iteration`, group by group (the
+// per-member launches of grid policy 2 need all members at once to fill the GPU)
+int ens_block(lbm_ensemble e, long long iteration, long long n)
+{
+	if (e->grid_policy == 2) {
+		for (long long s = 0; s < n; s++)
+			if (int rc = ens_launch(e, 0, e->count, iteration + s, false))
+				return rc;
+		return LBM_OK;
+	}
+	for (size_t k = 0; k + 1 < e->group0.size(); k++)
+		for (long long s = 0; s < n; s++)
+			if (int rc = ens_launch(e, e->group0[k], e->group0[k + 1], iteration + s, false))
+				return rc;
 	return LBM_OK;
 }
 
 int ens_build_graph(lbm_ensemble e)
 {
 	e->drop_graph();
-	const long long saved = e->iteration;
 	// resolve per-kernel launch facts outside of the capture
-	for (int parity = 0; parity < 2; parity++) {
-		e->iteration = parity;
-		if (int rc = ens_launch(e, false, true)) {
-			e->iteration = saved;
+	for (int parity = 0; parity < 2; parity++)
+		if (int rc = ens_launch(e, 0, e->count, parity, false, true))
 			return rc;
-		}
-	}
-	e->iteration = 0;  // the graph starts at an even step
 	cudaGraph_t graph = nullptr;
 	ENS_CUDA(cudaStreamBeginCapture(e->stream, cudaStreamCaptureModeThreadLocal));
-	int rc = LBM_OK;
-	for (int s = 0; s < lbm_ensemble_t::GRAPH_STEPS && rc == LBM_OK; s++)
-		rc = ens_launch(e, false);
+	const int rc = ens_block(e, 0, lbm_ensemble_t::GRAPH_STEPS);  // the graph starts at an even step
 	const cudaError_t end = cudaStreamEndCapture(e->stream, &graph);
-	e->iteration = saved;
 	if (rc != LBM_OK) {
 		if (graph)
 			cudaGraphDestroy(graph);
@@ -310,12 +352,16 @@ int ens_build_graph(lbm_ensemble e)
 
 int ens_plain_steps(lbm_ensemble e, long long n)
 {
-	while (n > 0 && (e->iteration % 2) != 0) {
-		if (int rc = ens_launch(e, false))
+	// to an even step ahead of a graph; a block of steps that no graph follows
+	// runs as one
+	const bool graphs = e->use_graphs && n - e->iteration % 2 >= lbm_ensemble_t::GRAPH_STEPS;
+	if (graphs && e->iteration % 2 != 0) {
+		if (int rc = ens_block(e, e->iteration, 1))
 			return rc;
+		e->iteration++;
 		n--;
 	}
-	if (e->use_graphs && n >= lbm_ensemble_t::GRAPH_STEPS) {
+	if (graphs && n >= lbm_ensemble_t::GRAPH_STEPS) {
 		if (!e->graph)
 			if (int rc = ens_build_graph(e))
 				return rc;
@@ -325,11 +371,9 @@ int ens_plain_steps(lbm_ensemble e, long long n)
 			n -= lbm_ensemble_t::GRAPH_STEPS;
 		}
 	}
-	while (n > 0) {
-		if (int rc = ens_launch(e, false))
-			return rc;
-		n--;
-	}
+	if (int rc = ens_block(e, e->iteration, n))
+		return rc;
+	e->iteration += n;
 	return LBM_OK;
 }
 
@@ -416,6 +460,7 @@ int lbm_ensemble_create(const lbm_ensemble_desc* d, lbm_ensemble* out)
 		p.eq = d->equilibrium;
 	}
 	e->pop_bytes = total;
+	build_groups(e);
 	auto cleanup = [&](int rc) {
 		lbm_ensemble_destroy(e);
 		return rc;
@@ -545,8 +590,9 @@ int lbm_ensemble_step(lbm_ensemble e, int64_t nsteps, int flags)
 		return rc;
 	e->sums_valid = false;
 	if (sums) {
-		if (int rc = ens_launch(e, true))
+		if (int rc = ens_launch(e, 0, e->count, e->iteration, true))
 			return rc;
+		e->iteration++;
 		// written straight into the mapped pinned buffer
 		ens_finish_kernel<<<e->count, 256, 0, e->stream>>>(e->partials, e->ntiles, e->tile0_dev, e->sums_mapped);
 		ENS_CUDA(cudaGetLastError());
