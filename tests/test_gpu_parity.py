@@ -283,6 +283,54 @@ def test_i16s_storage_is_the_stated_quantisation(pl, port):
     lat.close()
 
 
+@pytest.mark.parametrize("storage", ["F16S", "BF16S"])
+def test_16bit_storage_reads_back_the_stated_values(pl, storage):
+    """The value read back is h / s + w (F16S) or b + w (BF16S) in one rounding to
+    FP32, bit for bit, over every 16-bit pattern that a store can leave
+    (subnormals, the largest finite values, infinities and NaN among them)."""
+    import torch
+    X, Y, Z = 41, 40, 40
+    half = storage == "F16S"
+    nnz = np.array([0] + [1] * 6 + [2] * 12 + [3] * 8)
+    w = np.array([8 / 27, 2 / 27, 1 / 54, 1 / 216])[nnz].astype(np.float32).astype(np.float64).reshape(27, 1, 1, 1)
+    s = np.array([4.0, 16.0, 64.0, 256.0])[nnz].reshape(27, 1, 1, 1) if half else np.ones((27, 1, 1, 1))
+    pattern = torch.arange(X * Y * Z, dtype=torch.int32).remainder(65536).to(torch.int16)
+    stored = pattern.view(torch.float16 if half else torch.bfloat16).to(torch.float64).numpy().reshape(1, Z, Y, X)
+    lat = pl.LBM(X, Y, Z, viscosity=0.01, storage=getattr(pl, "STORE_" + storage), periodic=True)
+    view = lat.populations_tensor()
+    x0 = lat.device_view().x0
+    view[:, 1:-1, 1:-1, x0:x0 + X] = torch.from_numpy(stored).to(view.device).to(view.dtype)
+    torch.cuda.synchronize()
+    back = lat.get_populations(layout=pl.LAYOUT_INTERIOR, dtype=np.float32)
+    with np.errstate(over="ignore", invalid="ignore"):
+        want = (stored / s + w).astype(np.float32)  # FP64 holds the sum of 11 and 24 bits exactly
+    np.testing.assert_array_equal(back, want)
+    lat.close()
+
+
+@pytest.mark.parametrize("storage", ["F32", "F64"])
+@pytest.mark.parametrize("shape", [(8, 4, 4), (64, 64, 64), (65, 63, 67)])
+def test_fields_reach_the_host_whole(pl, storage, shape):
+    """The macro field and the populations against the device's own arrays, over
+    one thread's copy, several threads' and a last chunk that is not full."""
+    X, Y, Z = shape
+    lat = pl.LBM(X, Y, Z, viscosity=0.01, storage=getattr(pl, "STORE_" + storage), periodic=True)
+    lat.init_taylor_green(0.05)
+    lat.step(3, macro=True)
+    import torch
+    v = lat.device_view()
+    dt = torch.float32 if v.macro_elem_size == 4 else torch.float64
+    lat.synchronize()
+    dev = pl._wrap_device(v.macro, 4 * X * Y * Z, dt, 0).double().cpu().numpy().reshape(4, Z, Y, X)
+    for _ in range(2):
+        np.testing.assert_array_equal(lat.macro(), dev)
+    x0 = v.x0
+    pop = lat.populations_tensor()[:, 1:-1, 1:-1, x0:x0 + X].double().cpu().numpy()
+    np.testing.assert_array_equal(lat.get_populations(layout=pl.LAYOUT_INTERIOR), pop)
+    np.testing.assert_array_equal(lat.get_populations(layout=pl.LAYOUT_INTERIOR, dtype=np.float32), pop.astype(np.float32))
+    lat.close()
+
+
 @pytest.mark.parametrize("storage,tol", [("F32S", 1e-5), ("F16S", 2e-3), ("BF16S", 2e-2), ("F16SR", 2e-3),
                                          ("BF16SR", 2e-2), ("I16S", 2e-3)])
 def test_shifted_storage_follows_fp64(pl, storage, tol):

@@ -1,0 +1,138 @@
+// Device-to-host copies of fields into pageable memory (host_copy.h).
+#include "host_copy.h"
+
+#include <atomic>
+#include <cstring>
+#include <functional>
+#include <system_error>
+#include <thread>
+
+namespace lbm {
+
+namespace {
+
+struct Job
+{
+	HostCopy* c;
+	int device;
+	cudaStream_t stream;
+	const unsigned char* dev;
+	unsigned char* host;
+	int dev_size, host_size;
+	long long n, per_chunk, nchunks;
+	int threads;
+	std::atomic<int> error{cudaSuccess};
+};
+
+void deliver(const Job& j, const unsigned char* from, long long first, long long count)
+{
+	unsigned char* to = j.host + first * j.host_size;
+	if (j.dev_size == j.host_size) {
+		std::memcpy(to, from, (size_t) (count * j.dev_size));
+		return;
+	}
+	const float* f = reinterpret_cast<const float*>(from);
+	double* d = reinterpret_cast<double*>(to);
+	for (long long i = 0; i < count; i++)
+		d[i] = f[i];
+}
+
+// thread k takes chunks k, k + threads, ... through its two pinned chunks
+void work(Job& j, int k)
+{
+	cudaError_t e = cudaSetDevice(j.device);
+	auto issue = [&](long long chunk, int slot)
+	{
+		const long long first = chunk * j.per_chunk, count = j.n - first < j.per_chunk ? j.n - first : j.per_chunk;
+		e = cudaMemcpyAsync(j.c->pinned + (size_t) (2 * k + slot) * HostCopy::CHUNK, j.dev + first * j.dev_size,
+							(size_t) (count * j.dev_size), cudaMemcpyDeviceToHost, j.stream);
+		if (e == cudaSuccess)
+			e = cudaEventRecord(j.c->landed[2 * k + slot], j.stream);
+	};
+	int slot = 0;
+	if (e == cudaSuccess && k < j.nchunks)
+		issue(k, 0);
+	for (long long chunk = k; e == cudaSuccess && chunk < j.nchunks; chunk += j.threads) {
+		if (chunk + j.threads < j.nchunks)
+			issue(chunk + j.threads, slot ^ 1);
+		const cudaError_t s = cudaEventSynchronize(j.c->landed[2 * k + slot]);
+		if (e == cudaSuccess)
+			e = s;
+		if (e != cudaSuccess)
+			break;
+		const long long first = chunk * j.per_chunk;
+		deliver(j, j.c->pinned + (size_t) (2 * k + slot) * HostCopy::CHUNK, first, j.n - first < j.per_chunk ? j.n - first : j.per_chunk);
+		slot ^= 1;
+	}
+	if (e != cudaSuccess) {
+		cudaStreamSynchronize(j.stream);  // nothing of ours is in flight into the pinned chunks
+		j.error = (int) e;
+	}
+}
+
+}  // namespace
+
+void host_copy_free(HostCopy& c)
+{
+	if (c.pinned)
+		cudaFreeHost(c.pinned);
+	c.pinned = nullptr;
+	for (cudaEvent_t& ev : c.landed) {
+		if (ev)
+			cudaEventDestroy(ev);
+		ev = nullptr;
+	}
+}
+
+cudaError_t host_copy(HostCopy& c, int device, cudaStream_t stream, const void* dev, int dev_size, void* host, int host_size,
+					  long long n)
+{
+	if (n < 1)
+		return cudaStreamSynchronize(stream);
+	if (!c.pinned) {
+		cudaError_t e = cudaMallocHost((void**) &c.pinned, 2 * HostCopy::THREADS * HostCopy::CHUNK);
+		for (cudaEvent_t& ev : c.landed)
+			if (e == cudaSuccess)
+				e = cudaEventCreateWithFlags(&ev, cudaEventDisableTiming);
+		if (e != cudaSuccess) {
+			host_copy_free(c);
+			return e;
+		}
+	}
+	Job j;
+	j.c = &c;
+	j.device = device;
+	j.stream = stream;
+	j.dev = (const unsigned char*) dev;
+	j.host = (unsigned char*) host;
+	j.dev_size = dev_size;
+	j.host_size = host_size;
+	j.n = n;
+	j.per_chunk = (long long) HostCopy::CHUNK / dev_size;
+	j.nchunks = (n + j.per_chunk - 1) / j.per_chunk;
+	// a thread is worth starting for a few chunks
+	j.threads = j.nchunks >= 4 * HostCopy::THREADS ? HostCopy::THREADS : 1;
+	std::thread helpers[HostCopy::THREADS - 1];
+	int started = 0;
+	if (j.threads > 1) {
+		// the stream's work first: the helpers start when there is something to move
+		const cudaError_t e = cudaStreamSynchronize(stream);
+		if (e != cudaSuccess)
+			return e;
+		try {
+			for (; started < HostCopy::THREADS - 1; started++)
+				helpers[started] = std::thread(work, std::ref(j), started + 1);
+		}
+		catch (const std::system_error&) {
+			// no more threads to be had: this one takes the others' shares below
+		}
+	}
+	for (int k = 0; k < j.threads; k++)
+		if (k == 0 || k > started)
+			work(j, k);
+	for (int k = 0; k < started; k++)
+		helpers[k].join();
+	return (cudaError_t) j.error.load();
+}
+
+}  // namespace lbm

@@ -9,6 +9,7 @@
 #include <cuda_runtime.h>
 
 #include "../../include/tnl_lbm_b200.h"
+#include "host_copy.h"
 #include "launch.h"
 
 namespace lbm {
@@ -115,6 +116,7 @@ struct lbm_lattice
 	lbm::AdjointState* adjoint = nullptr;	 // checkpoints of lbm_adjoint_forward
 	lbm::AdeState* ade = nullptr;			 // coupled D3Q7 scalar, or null
 	bool distributed_z = false;				 // a slab of a lattice split along z (lbm_set_distributed_z)
+	lbm::HostCopy host_copy;				 // staging of the fields handed to the caller
 	cudaEvent_t halo_ev = nullptr;			 // ordering of halo copies against this lattice's stream
 	static constexpr int GRAPH_STEPS = 16;
 

@@ -517,6 +517,7 @@ int lbm_destroy(lbm_handle h)
 	if (h->stream)
 		cudaStreamSynchronize(h->stream);
 	h->drop_graph();
+	lbm::host_copy_free(h->host_copy);
 	lbm::adjoint_free(h->adjoint);
 	lbm::ade_free(h->ade);
 	cudaFree(h->g.f);
@@ -842,9 +843,11 @@ int lbm_get_populations(lbm_handle h, void* host, int layout, int dtype)
 		cudaFreeAsync(dev, h->stream);
 		return fail(LBM_ERR_CUDA, "pack failed: %s", cudaGetErrorString(e));
 	}
-	LBM_CUDA(cudaMemcpyAsync(host, dev, bytes, cudaMemcpyDeviceToHost, h->stream));
+	const int value = dtype == 0 ? 8 : 4;
+	const cudaError_t c =
+		lbm::host_copy(h->host_copy, h->d.device, h->stream, dev, value, host, value, (long long) dense_count(h, layout));
 	cudaFreeAsync(dev, h->stream);
-	LBM_CUDA(cudaStreamSynchronize(h->stream));
+	LBM_CUDA(c);
 	return LBM_OK;
 }
 
@@ -948,18 +951,8 @@ int lbm_get_macro(lbm_handle h, double* host)
 		return fail(LBM_ERR_INVALID, "null output");
 	if (!h->macro_valid)
 		return fail(LBM_ERR_INVALID, "no macro field: run lbm_step with LBM_STEP_MACRO first");
-	const size_t n = 4 * (size_t) h->sites();
-	if (h->ops->compute_size == 8) {
-		LBM_CUDA(cudaMemcpyAsync(host, h->macro, n * 8, cudaMemcpyDeviceToHost, h->stream));
-		LBM_CUDA(cudaStreamSynchronize(h->stream));
-	}
-	else {
-		std::vector<float> tmp(n);
-		LBM_CUDA(cudaMemcpyAsync(tmp.data(), h->macro, n * 4, cudaMemcpyDeviceToHost, h->stream));
-		LBM_CUDA(cudaStreamSynchronize(h->stream));
-		for (size_t i = 0; i < n; i++)
-			host[i] = tmp[i];
-	}
+	const int cs = h->ops->compute_size;
+	LBM_CUDA(lbm::host_copy(h->host_copy, h->d.device, h->stream, h->macro, cs, host, 8, 4 * h->sites()));
 	return LBM_OK;
 }
 
@@ -1186,19 +1179,8 @@ int lbm_get_statistics(lbm_handle h, double* out, int64_t* count)
 		return fail(LBM_ERR_INVALID, "statistics are not enabled (lbm_set_statistics)");
 	if (!out || !count)
 		return fail(LBM_ERR_INVALID, "null output");
-	const size_t n = (size_t) 9 * h->sites();
 	const int cs = h->ops->compute_size;
-	if (cs == 8) {
-		LBM_CUDA(cudaMemcpyAsync(out, h->stats, n * 8, cudaMemcpyDeviceToHost, h->stream));
-		LBM_CUDA(cudaStreamSynchronize(h->stream));
-	}
-	else {
-		std::vector<float> tmp(n);
-		LBM_CUDA(cudaMemcpyAsync(tmp.data(), h->stats, n * 4, cudaMemcpyDeviceToHost, h->stream));
-		LBM_CUDA(cudaStreamSynchronize(h->stream));
-		for (size_t i = 0; i < n; i++)
-			out[i] = tmp[i];
-	}
+	LBM_CUDA(lbm::host_copy(h->host_copy, h->d.device, h->stream, h->stats, cs, out, 8, 9 * h->sites()));
 	*count = h->stats_count;
 	return LBM_OK;
 }

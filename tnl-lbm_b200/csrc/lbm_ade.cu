@@ -379,7 +379,8 @@ int lbm_ade_get_populations(lbm_handle h, void* host, int layout, int dtype)
 	void* dev = nullptr;
 	ADE_CUDA(cudaMallocAsync(&dev, bytes, h->stream));
 	int rc = convert(h, dev, dtype, layout, true);
-	if (rc == LBM_OK && cudaMemcpyAsync(host, dev, bytes, cudaMemcpyDeviceToHost, h->stream) != cudaSuccess)
+	const int value = dtype == 0 ? 8 : 4;
+	if (rc == LBM_OK && lbm::host_copy(h->host_copy, h->d.device, h->stream, dev, value, host, value, dense_count(h, layout)) != cudaSuccess)
 		rc = efail(LBM_ERR_CUDA, "scalar population copy failed");
 	cudaFreeAsync(dev, h->stream);
 	ADE_CUDA(cudaStreamSynchronize(h->stream));
@@ -394,16 +395,7 @@ int lbm_ade_get_phi(lbm_handle h, double* host)
 		return efail(LBM_ERR_INVALID, "null output");
 	if (!h->macro_valid || !h->ade->phi_valid)
 		return efail(LBM_ERR_INVALID, "no scalar field: run lbm_step with LBM_STEP_MACRO first");
-	const size_t n = (size_t) h->sites();
-	const size_t cs = (size_t) h->ops->compute_size;
-	std::vector<unsigned char> tmp(n * cs);
-	ADE_CUDA(cudaMemcpyAsync(tmp.data(), h->ade->phi_buf, n * cs, cudaMemcpyDeviceToHost, h->stream));
-	ADE_CUDA(cudaStreamSynchronize(h->stream));
-	if (cs == 8)
-		std::memcpy(host, tmp.data(), n * 8);
-	else
-		for (size_t i = 0; i < n; i++)
-			host[i] = ((const float*) tmp.data())[i];
+	ADE_CUDA(lbm::host_copy(h->host_copy, h->d.device, h->stream, h->ade->phi_buf, h->ops->compute_size, host, 8, h->sites()));
 	return LBM_OK;
 }
 

@@ -20,6 +20,7 @@
 
 #include "../../include/tnl_lbm_b200.h"
 #include "host_common.h"
+#include "host_copy.h"
 #include "launch.h"
 
 namespace lbm {
@@ -103,6 +104,7 @@ struct lbm_ensemble_t
 	bool sums_valid = false;
 	long long iteration = 0;
 	cudaGraphExec_t graph = nullptr;
+	lbm::HostCopy host_copy;  // staging of the populations handed to the caller
 	// grid policy 2: one stream per lane, members round-robin over the lanes
 	std::vector<cudaStream_t> lanes;
 	std::vector<cudaEvent_t> joins;
@@ -491,6 +493,7 @@ int lbm_ensemble_destroy(lbm_ensemble e)
 	if (e->stream)
 		cudaStreamSynchronize(e->stream);
 	e->drop_graph();
+	lbm::host_copy_free(e->host_copy);
 	e->free_tiles();
 	cudaFree(e->pops);
 	cudaFreeHost(e->sums_host);
@@ -569,9 +572,11 @@ int lbm_ensemble_get_populations(lbm_ensemble e, int member, void* host, int lay
 		cudaFreeAsync(dev, e->stream);
 		return efail(LBM_ERR_CUDA, "pack failed: %s", cudaGetErrorString(err));
 	}
-	ENS_CUDA(cudaMemcpyAsync(host, dev, bytes, cudaMemcpyDeviceToHost, e->stream));
+	const int value = dtype == 0 ? 8 : 4;
+	const cudaError_t c = lbm::host_copy(e->host_copy, e->device, e->stream, dev, value, host, value,
+										 (long long) dense_count(e->g[member], layout));
 	cudaFreeAsync(dev, e->stream);
-	ENS_CUDA(cudaStreamSynchronize(e->stream));
+	ENS_CUDA(c);
 	return LBM_OK;
 }
 
