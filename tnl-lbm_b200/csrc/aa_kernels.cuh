@@ -331,18 +331,20 @@ __device__ __forceinline__ void warp_reduce_store(const double (&v)[NRED], doubl
 }
 
 // Consecutive steps are programmatic dependent launches (launch_dependent,
-// launch.h).  launch_dependents lets the next step's grid (or the finish kernel
-// of the sums) be scheduled once every block of this grid has started;
-// await_predecessor, the first thing a step kernel does, returns when the grid
-// before it has completed and its writes are visible.  The launch latency and
-// the start of the blocks then lie inside the step before: 64^3 Taylor-Green
-// vortex 9.1 -> 8.5 us a step, duct 171x45x45 12.0 -> 11.5, 96x48x40 8.4 -> 8.0,
-// FP64 A-B 100x32x32 8.1 -> 7.5, 512x128x128 283.6 -> 282.4.  (Waiting only
-// ahead of the population loads gains no more and costs FP64 A-B 1.5 % and
-// SRT 2 % through the compiler's order of the loads.)
+// launch.h).  await_predecessor, the first thing a step kernel does, returns when
+// the grid before it has completed and its writes are visible; launch_dependents,
+// ahead of a site's stores, lets the next grid be scheduled once every block of
+// this one has come that far.  The launch latency then lies under the stores: us
+// a step, graph replay and (ten steps launched one by one): 24^3 Taylor-Green
+// vortex 2.6 -> 2.2 (5.4 -> 4.6), 32^3 3.3 -> 3.0 (6.2 -> 4.6), 64^3 9.0 -> 8.6
+// (11.9 -> 9.8), 96x96x64 17.7 -> 17.3 (20.6 -> 18.6), duct 171x45x45 11.8 -> 11.5,
+// 512x128x128 285.4 -> 283.8.  Let go at its start instead, a grid of a fraction
+// of a wave has its successor's blocks beside it, which then lie unevenly over
+// the SMs (48^3 5.5 -> 6.5).  Waiting only ahead of the loads gains no more and
+// costs FP64 A-B 1.5 % through the compiler's order of the loads.
 __device__ __forceinline__ void launch_dependents()
 {
-	asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+	asm volatile("griddepcontrol.launch_dependents;");
 }
 __device__ __forceinline__ void await_predecessor()
 {
@@ -461,6 +463,7 @@ __device__ __forceinline__ void aa_step_site(const StepArgs<typename S::T, typen
 	if (write) {
 		if (coll)
 			collide(s);
+		launch_dependents();
 		aa_write<S, ODD>(a.f, a.sq, base, o, s.f);
 	}
 }
@@ -469,7 +472,6 @@ template <typename S, int COLL, int CUMF, bool ODD, bool GENERAL, bool OUT, int 
 __global__ void __launch_bounds__(128, MINB) aa_step_kernel(const StepArgs<typename S::T, typename S::R> a)
 {
 	using R = typename S::R;
-	launch_dependents();
 	await_predecessor();
 	aa_step_site<S, ODD, GENERAL, OUT>(a, [&](Site<R>& s) { collide<R, COLL, CUMF>(s, a.p); });
 }

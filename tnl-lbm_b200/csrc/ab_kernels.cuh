@@ -129,7 +129,6 @@ __global__ void __launch_bounds__(128, MINB)
 	ab_step_kernel(const StepArgs<typename S::T, typename S::R> a, typename S::T* __restrict__ fout)
 {
 	using R = typename S::R;
-	launch_dependents();
 	await_predecessor();
 	const int x = blockIdx.x * blockDim.x + threadIdx.x;
 	const int y = blockIdx.y * blockDim.y + threadIdx.y;
@@ -161,6 +160,7 @@ __global__ void __launch_bounds__(128, MINB)
 	if (write) {
 		if (coll)
 			collide<R, COLL, CUMF>(s, a.p);
+		launch_dependents();
 		static_for<27>(
 			[&](auto Qc)
 			{

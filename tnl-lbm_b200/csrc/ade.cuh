@@ -318,6 +318,7 @@ __device__ __forceinline__ void ade_site_update(const StepArgs<typename S::T, ty
 	if (write) {
 		if (coll)
 			collide<R, COLL, CUMF>(s, a.p);
+		launch_dependents();
 		aa_write<S, ODD>(a.f, a.sq, base, o, s.f);
 	}
 	if (!active)
@@ -349,7 +350,6 @@ template <typename S, int COLL, int CUMF, bool ODD, bool GENERAL, bool OUT, int 
 __global__ void __launch_bounds__(128, MINB)
 	ade_step_kernel(const StepArgs<typename S::T, typename S::R> a, const AdeArgs<typename S::R> d)
 {
-	launch_dependents();
 	await_predecessor();
 	ade_site_update<S, COLL, CUMF, ODD, GENERAL, OUT>(a, d, blockIdx.x * blockDim.x + threadIdx.x,
 													  blockIdx.y * blockDim.y + threadIdx.y, blockIdx.z);

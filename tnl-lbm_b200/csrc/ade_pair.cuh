@@ -103,6 +103,7 @@ __device__ __forceinline__ void ade_pair_update(const StepArgs<typename S::T, fl
 	if (!act)
 		return;
 	collide_cumulant<F2, CUMF>(s, p2);
+	launch_dependents();
 	pair_write_at<S, ODD>(at, ps, s);
 	// the scalar, advected with the pair's flow velocity (unchanged by the collision)
 	const F2 phi = ade_phi(g);
@@ -118,7 +119,6 @@ __global__ void __launch_bounds__(128, MINB)
 						 const PairSlots psd, const PairRows pr, const AdeArgs<float> d, const uint8_t* __restrict__ groups,
 						 const unsigned* __restrict__ work, const unsigned long long* __restrict__ rest, long long nrest)
 {
-	launch_dependents();
 	await_predecessor();
 	const unsigned w = work[blockIdx.x];
 	if (w & PAIR_WORK_REST) {

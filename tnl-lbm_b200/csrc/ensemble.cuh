@@ -51,7 +51,6 @@ __global__ void __launch_bounds__(TPB, MINB)
 	__shared__ EnsMember<T, R> M;
 	constexpr int WORDS = (int) (sizeof(EnsMember<T, R>) / 4);
 	static_assert(sizeof(EnsMember<T, R>) % 4 == 0 && WORDS <= TPB, "member entry size");
-	launch_dependents();
 	await_predecessor();
 	int cur = -1;
 	for (long long t = tile_begin + blockIdx.x; t < tile_end; t += gridDim.x) {
@@ -79,6 +78,7 @@ __global__ void __launch_bounds__(TPB, MINB)
 			aa_read<S, ODD>(f, sq, base, o, s.f);
 			density_velocity(s, p);
 			collide<R, COLL, CUMF>(s, p);
+			launch_dependents();
 			aa_write<S, ODD>(f, sq, base, o, s.f);
 			if constexpr (OUT) {
 				const double rho = (double) s.rho, vx = (double) s.vx, vy = (double) s.vy, vz = (double) s.vz;
@@ -136,7 +136,6 @@ __global__ void __launch_bounds__(128, MINB)
 	__shared__ PairSlots ps;
 	constexpr int WORDS = (int) (sizeof(EnsMember<T, float>) / 4);
 	static_assert(sizeof(EnsMember<T, float>) % 4 == 0 && WORDS <= 128, "member entry size");
-	launch_dependents();
 	await_predecessor();
 	int cur = -1;
 	for (long long t = tile_begin + blockIdx.x; t < tile_end; t += gridDim.x) {
@@ -180,6 +179,7 @@ __global__ void __launch_bounds__(128, MINB)
 				}
 			}
 			collide<F2, COLL, CUMF>(s, M.p2);
+			launch_dependents();
 			pair_write_at<S, ODD>(at, ps, s);
 		}
 		if constexpr (OUT) {

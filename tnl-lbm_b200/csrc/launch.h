@@ -10,7 +10,7 @@
 namespace lbm {
 
 // Launches a step kernel as a programmatic dependent of the kernel before it on
-// the stream: its blocks are scheduled while that kernel's last ones run and
+// the stream: its blocks are scheduled while that kernel's last ones store and
 // wait in await_predecessor (aa_kernels.cuh).  After anything but a kernel (a
 // copy, a wait on an event) it starts as an ordinary launch.  Only for kernels
 // whose every thread begins with await_predecessor: one that did not wait could

@@ -622,6 +622,7 @@ __device__ __forceinline__ void pair_update(const StepArgs<typename S::T, float>
 		// the work kernel: populations first, sums after the stores
 		if (act) {
 			C::template collision<F2>(s, p2);
+			launch_dependents();
 			pair_write_at<S, ODD>(at, ps, s);
 		}
 		pair_outputs(a, act, act, site, s, slot, nslots);
@@ -641,6 +642,7 @@ __device__ __forceinline__ void pair_update(const StepArgs<typename S::T, float>
 	if (!act)
 		return;
 	C::template collision<F2>(s, p2);
+	launch_dependents();
 	pair_write_at<S, ODD, RAGGED>(at, ps, s);
 }
 
@@ -704,6 +706,7 @@ __device__ __forceinline__ void rest_update(const StepArgs<typename S::T, float>
 		return;
 	if (coll)
 		C::template collision<float>(s, a.p);
+	launch_dependents();
 	aa_write<S, ODD>(a.f, a.sq, base, o, s.f);
 }
 
@@ -713,7 +716,6 @@ template <typename S, typename C, bool ODD, bool OUT, bool RAGGED, int MINB>
 __global__ void __launch_bounds__(128, MINB) aa_pair_kernel(const StepArgs<typename S::T, float> a, const CollParams<F2> p2,
 															 const PairSlots ps, const PairRows pr, long long red_slots)
 {
-	launch_dependents();
 	await_predecessor();
 	const long long slot = (long long) blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
 	int x, y, z;
@@ -734,7 +736,6 @@ __global__ void __launch_bounds__(128, MINB)
 						const uint8_t* __restrict__ groups, const unsigned* __restrict__ work,
 						const unsigned long long* __restrict__ rest, long long nrest)
 {
-	launch_dependents();
 	await_predecessor();
 	const unsigned w = work[blockIdx.x];
 	const long long slot = (long long) blockIdx.x * 4 + (threadIdx.x >> 5);
