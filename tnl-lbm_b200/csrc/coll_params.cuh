@@ -33,6 +33,12 @@ inline CollParams<R> make_coll_params(const CollParamsD& d)
 	p.c43 = (R) (2.0 / 3.0 * g * d.A);
 	p.c45 = (R) (-4.0 / 3.0 * g * d.A);
 	p.cB = (R) (-1.0 / 3.0 * g * d.B);
+	p.l3 = (R) (0.5 * 0.01 * (1.0 - d.w3));
+	p.l4 = (R) (0.5 * 0.01 * (1.0 - d.w4));
+	p.l5 = (R) (0.01 * (1.0 - d.w5));
+	p.kA = (R) (0.5 * w1 * (2.0 / 3.0 * g * d.A));
+	p.k45 = (R) (0.5 * w1 * (-4.0 / 3.0 * g * d.A));
+	p.kB = (R) (-3.0 * w1 * (-1.0 / 3.0 * g * d.B));
 	p.inv_tau = (R) (1.0 / d.tau);
 	p.srt_force = (R) (1.0 - 0.5 / d.tau);
 	p.bgk_force = (R) (1.0 - 0.5 * w1);

@@ -50,15 +50,15 @@ __global__ void __launch_bounds__(TPB, MINB)
 	// read where they are used instead of occupying registers
 	__shared__ EnsMember<T, R> M;
 	constexpr int WORDS = (int) (sizeof(EnsMember<T, R>) / 4);
-	static_assert(sizeof(EnsMember<T, R>) % 4 == 0 && WORDS <= TPB, "member entry size");
+	static_assert(sizeof(EnsMember<T, R>) % 4 == 0, "member entry size");
 	await_predecessor();
 	int cur = -1;
 	for (long long t = tile_begin + blockIdx.x; t < tile_end; t += gridDim.x) {
 		const int m = tile_member[t];
 		if (m != cur) {
 			__syncthreads();  // every thread is done with the previous entry
-			if ((int) threadIdx.x < WORDS)
-				reinterpret_cast<unsigned*>(&M)[threadIdx.x] = reinterpret_cast<const unsigned*>(members + m)[threadIdx.x];
+			for (int w = (int) threadIdx.x; w < WORDS; w += TPB)
+				reinterpret_cast<unsigned*>(&M)[w] = reinterpret_cast<const unsigned*>(members + m)[w];
 			__syncthreads();
 			cur = m;
 		}

@@ -73,6 +73,10 @@ __device__ __forceinline__ F2 fma2(F2 a, F2 b, F2 c)
 {
 	return F2(__ffma2_rn(a.v, b.v, c.v));
 }
+__device__ __forceinline__ F2 fmadd(F2 a, F2 b, F2 c)
+{
+	return fma2(a, b, c);
+}
 __device__ __forceinline__ F2 fabs(F2 a)
 {
 	return F2(fabsf(a.v.x), fabsf(a.v.y));
