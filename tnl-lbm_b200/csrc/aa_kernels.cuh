@@ -460,6 +460,10 @@ __device__ __forceinline__ void aa_step_site(const StepArgs<typename S::T, typen
 	}
 	if constexpr (OUT)
 		step_outputs(a, active, site, s);
+	else if constexpr (sizeof(R) == 8)
+		// keeps the collision after the loads: mixed, the FP64 step takes 168
+		// registers and spills, apart 124
+		__syncwarp();
 	if (write) {
 		if (coll)
 			collide(s);

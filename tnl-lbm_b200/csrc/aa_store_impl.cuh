@@ -25,17 +25,17 @@ namespace lbm {
 // (OUT) needs no more registers than the plain step: its outputs are written
 // before the collision.  The FP64 kernels need twice the registers per value.
 //
-// FP64 arithmetic: 4 blocks (128 registers, up to 24 bytes of spills) for
-// MRT and the default and anti-aliased cumulant, 3 (168 registers, up to 68
-// bytes) for SRT, BGK and the Geier-2017 cumulant, which spill 140-500 bytes
-// at 4.  Against 2 blocks (the full 256 registers, of which these kernels use
-// 110-150), duct: cumulant 14.5 -> 15.3, SRT 11.7 -> 13.6, BGK 13.1 -> 14.5,
-// MRT 14.3 -> 15.2 GLUPS; 256^3 Taylor-Green vortex (Geier 2017) 10.7 -> 12.9.
+// FP64 arithmetic: 4 blocks (128 registers, at most 48 bytes of spills).  With the
+// warp sync between loads and collision (aa_step_site) the kernels take 110-142
+// registers; without it 168 and spills, at 3 blocks for SRT, BGK and the
+// Geier-2017 cumulant.  B200, us a step: Taylor-Green vortex (Geier 2017) 64^3 18.0
+// -> 16.6, 128^3 154.5 -> 146.1; duct 256x96x96 SRT 159 -> 155, BGK 162 -> 155,
+// cumulant and MRT 155 (432 bytes a site through HBM at 6.6 TB/s).
 template <typename R, int COLL, int CUMF, bool ODD, bool GENERAL, bool OUT>
 constexpr int direct_minb()
 {
 	if (sizeof(R) == 8)
-		return COLL == COLL_SRT || COLL == COLL_BGK || (COLL == COLL_CUM && (CUMF & CUM_2017)) ? 3 : 4;
+		return 4;
 	if (!ODD && GENERAL)
 		return 6;  // the even general step keeps no neighbour offsets: 80 registers
 	if (COLL == COLL_CUM || COLL == COLL_MRT)
@@ -51,15 +51,14 @@ constexpr int ade_minb()
 	return sizeof(R) == 8 ? 2 : direct_minb<R, COLL, CUMF, ODD, GENERAL, OUT>();
 }
 
-// resident blocks of the A-B step; its observation variant spills at 5.  In
-// FP64, 3 blocks (168 registers, 56-144 bytes of spills; the step uses about
-// 200 at 2): duct cumulant 11.8 -> 13.8, SRT 11.6 -> 13.7 GLUPS
+// resident blocks of the A-B step; its FP32 observation variant spills at 5.
+// FP64 as the A-A step, with the same warp sync (168 registers and 56-144 bytes
+// of spills without it, at 3 blocks): duct 256x96x96 cumulant 166.6 -> 154.5 us a
+// step.
 template <typename R, int COLL, int CUMF, bool OUT>
 constexpr int ab_minb()
 {
-	if (sizeof(R) == 8)
-		return 3;
-	if (OUT)
+	if (sizeof(R) == 8 || OUT)
 		return 4;
 	return direct_minb<R, COLL, CUMF, true, true, false>();
 }

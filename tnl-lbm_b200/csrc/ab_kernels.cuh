@@ -157,6 +157,8 @@ __global__ void __launch_bounds__(128, MINB)
 	}
 	if constexpr (OUT)
 		step_outputs(a, active, site, s);
+	else if constexpr (sizeof(R) == 8)
+		__syncwarp();  // as aa_step_site
 	if (write) {
 		if (coll)
 			collide<R, COLL, CUMF>(s, a.p);
