@@ -119,8 +119,8 @@ __global__ void __launch_bounds__(128, MINB)
 						 const PairSlots psd, const PairRows pr, const AdeArgs<float> d, const uint8_t* __restrict__ groups,
 						 const unsigned* __restrict__ work, const unsigned long long* __restrict__ rest, long long nrest)
 {
+	const unsigned w = work[blockIdx.x];  // no step writes the list
 	await_predecessor();
-	const unsigned w = work[blockIdx.x];
 	if (w & PAIR_WORK_REST) {
 		const long long i = (long long) (w & ~PAIR_WORK_REST) * 128 + threadIdx.x;
 		// threads past the list take x = X: no site, but every thread of the

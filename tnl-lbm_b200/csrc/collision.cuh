@@ -496,43 +496,74 @@ __device__ __forceinline__ R inv_rho_or_one(const Site<R>& s)
 	return s.rho == R(0) ? R(1) : s.ir;
 }
 
-// Textbook BGK (col_srt.h:14-105).  The equilibrium of a direction is formed and
-// used at once, and the second-order one for two opposite directions together
-// (even part a, odd part b); the forcing 3 (c - u).F / rho feq is linear in c, its
-// factor k0 + c.k.  The population itself is rounded once.  (With the 27
-// equilibria in an array first, the packed kernel spilled 56-170 bytes.)  B200,
-// us a step: duct 512x128x128 FP32 on the two-site kernel 318 -> 289, 256x96x96 FP64
-// 171 -> 159.
+// Guo-like forcing term S_q = 3 (c_q - u).F / rho (col_srt.h:22-48)
+template <int Q, typename R>
+__device__ __forceinline__ R force_term(const Site<R>& s, const CollParams<R>& p, R irho)
+{
+	return R(3) * ((R(cx(Q)) - s.vx) * p.fx + (R(cy(Q)) - s.vy) * p.fy + (R(cz(Q)) - s.vz) * p.fz) * irho;
+}
+
+// relaxation and forcing of one direction; the population is rounded once
 template <typename R>
 __device__ __forceinline__ void relax(R& f, R feq, R rate, R k)
 {
 	f = f + fmadd(feq - f, rate, feq * k);
 }
+
+// Textbook BGK (col_srt.h:14-105).  FP64 and the packed pairs form the equilibrium
+// of a direction where it is used, the second-order one for two opposite
+// directions together (its even and odd part; each direction's product with the
+// weight is rounded by itself, or the density errors of a pair would add up), and
+// the forcing 3 (c - u).F / rho feq as linear in c, its factor k0 + c.k: with the 27
+// equilibria in an array first the packed kernel spilled 56-170 bytes.  B200, us a
+// step: duct 512x128x128 FP32 on the two-site kernel 318 -> 289, 256x96x96 FP64
+// 171 -> 159.  One site in FP32 keeps the reference's order of operations: nothing
+// spills there, and the adjoint's objective in FP32 is nearer to FP64 with it.
 template <typename R>
 __device__ __forceinline__ void collide_srt(Site<R>& s, const CollParams<R>& p)
 {
-	const R rho = s.rho, vx = s.vx, vy = s.vy, vz = s.vz;
-	const R g = R(3) * (p.srt_force * inv_rho_or_one(s));
-	const R kx = g * p.fx, ky = g * p.fy, kz = g * p.fz;
-	const R k0 = -fmadd(vx, kx, fmadd(vy, ky, vz * kz));
-	if (p.eq == EQ_INV_CUM) {
-		const R vx3 = R(3) * vx * vx, vy3 = R(3) * vy * vy, vz3 = R(3) * vz * vz;
-		each_direction([&](auto Qc) {
-			constexpr int q = decltype(Qc)::value;
-			relax(s.f[q], eq_inv_cum<q>(rho, vx, vy, vz, vx3, vy3, vz3), p.inv_tau, along<q>(kx, ky, kz) + k0);
-		});
+	if constexpr (std::is_same<R, float>::value) {
+		R feq[27];
+		set_equilibrium(feq, p.eq, s.rho, s.vx, s.vy, s.vz);
+		const R irho = inv_rho_or_one(s);
+		each_direction(
+			[&](auto Qc)
+			{
+				constexpr int q = decltype(Qc)::value;
+				s.f[q] += (feq[q] - s.f[q]) * p.inv_tau + p.srt_force * force_term<q>(s, p, irho) * feq[q];
+			}
+		);
 	}
 	else {
-		const R base = fmadd(R(-1.5), fmadd(vx, vx, fmadd(vy, vy, vz * vz)), R(1));
-		relax(s.f[ZZZ], (R(weight(ZZZ)) * rho) * base, p.inv_tau, k0);
-		each_pair([&](auto Qc) {
-			constexpr int q = decltype(Qc)::value, m = opp(q);
-			const R wr = R(weight(q)) * rho;
-			const R cu = along<q>(vx, vy, vz), ck = along<q>(kx, ky, kz);
-			const R a = wr * fmadd(R(4.5) * cu, cu, base), b = wr * (R(3) * cu);
-			relax(s.f[q], a + b, p.inv_tau, k0 + ck);
-			relax(s.f[m], a - b, p.inv_tau, k0 - ck);
-		});
+		const R rho = s.rho, vx = s.vx, vy = s.vy, vz = s.vz;
+		const R g = R(3) * (p.srt_force * inv_rho_or_one(s));
+		const R kx = g * p.fx, ky = g * p.fy, kz = g * p.fz;
+		const R k0 = -fmadd(vx, kx, fmadd(vy, ky, vz * kz));
+		if (p.eq == EQ_INV_CUM) {
+			const R vx3 = R(3) * vx * vx, vy3 = R(3) * vy * vy, vz3 = R(3) * vz * vz;
+			each_direction(
+				[&](auto Qc)
+				{
+					constexpr int q = decltype(Qc)::value;
+					relax(s.f[q], eq_inv_cum<q>(rho, vx, vy, vz, vx3, vy3, vz3), p.inv_tau, along<q>(kx, ky, kz) + k0);
+				}
+			);
+		}
+		else {
+			const R base = fmadd(R(-1.5), fmadd(vx, vx, fmadd(vy, vy, vz * vz)), R(1));
+			relax(s.f[ZZZ], (R(weight(ZZZ)) * rho) * base, p.inv_tau, k0);
+			each_pair(
+				[&](auto Qc)
+				{
+					constexpr int q = decltype(Qc)::value, m = opp(q);
+					const R wr = R(weight(q)) * rho;
+					const R cu = along<q>(vx, vy, vz), ck = along<q>(kx, ky, kz);
+					const R even = fmadd(R(4.5) * cu, cu, base), odd = R(3) * cu;
+					relax(s.f[q], wr * (even + odd), p.inv_tau, k0 + ck);
+					relax(s.f[m], wr * (even - odd), p.inv_tau, k0 - ck);
+				}
+			);
+		}
 	}
 }
 

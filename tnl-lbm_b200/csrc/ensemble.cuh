@@ -51,7 +51,6 @@ __global__ void __launch_bounds__(TPB, MINB)
 	__shared__ EnsMember<T, R> M;
 	constexpr int WORDS = (int) (sizeof(EnsMember<T, R>) / 4);
 	static_assert(sizeof(EnsMember<T, R>) % 4 == 0, "member entry size");
-	await_predecessor();
 	int cur = -1;
 	for (long long t = tile_begin + blockIdx.x; t < tile_end; t += gridDim.x) {
 		const int m = tile_member[t];
@@ -62,6 +61,7 @@ __global__ void __launch_bounds__(TPB, MINB)
 			__syncthreads();
 			cur = m;
 		}
+		await_predecessor();  // of the first tile's loads on; no step writes the tables
 		const unsigned i = (unsigned) ((t - M.tile0) * TPB) + threadIdx.x;
 		double red[NRED] = {0, 0, 0, 0, 0, 0};
 		if (i < (unsigned) M.n) {
@@ -136,7 +136,6 @@ __global__ void __launch_bounds__(128, MINB)
 	__shared__ PairSlots ps;
 	constexpr int WORDS = (int) (sizeof(EnsMember<T, float>) / 4);
 	static_assert(sizeof(EnsMember<T, float>) % 4 == 0 && WORDS <= 128, "member entry size");
-	await_predecessor();
 	int cur = -1;
 	for (long long t = tile_begin + blockIdx.x; t < tile_end; t += gridDim.x) {
 		const int m = tile_member[t];
@@ -149,6 +148,7 @@ __global__ void __launch_bounds__(128, MINB)
 			__syncthreads();
 			cur = m;
 		}
+		await_predecessor();  // of the first tile's loads on; no step writes the tables
 		const unsigned i = (unsigned) ((t - M.tile0) * 256) + 2 * threadIdx.x;
 		const bool act = i < (unsigned) M.n;
 		Site<F2> s;

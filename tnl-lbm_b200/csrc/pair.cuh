@@ -740,8 +740,8 @@ __global__ void __launch_bounds__(128, MINB)
 						const uint8_t* __restrict__ groups, const unsigned* __restrict__ work,
 						const unsigned long long* __restrict__ rest, long long nrest)
 {
+	const unsigned w = work[blockIdx.x];  // no step writes the list
 	await_predecessor();
-	const unsigned w = work[blockIdx.x];
 	const long long slot = (long long) blockIdx.x * 4 + (threadIdx.x >> 5);
 	const long long nslots = (long long) gridDim.x * 4;
 	if (w & PAIR_WORK_REST) {
