@@ -24,11 +24,11 @@ struct Job
 	std::atomic<int> error{cudaSuccess};
 };
 
-void deliver(const Job& j, const unsigned char* from, long long first, long long count)
+void deliver(const unsigned char* from, int dev_size, unsigned char* host, int host_size, long long first, long long count)
 {
-	unsigned char* to = j.host + first * j.host_size;
-	if (j.dev_size == j.host_size) {
-		std::memcpy(to, from, (size_t) (count * j.dev_size));
+	unsigned char* to = host + first * host_size;
+	if (dev_size == host_size) {
+		std::memcpy(to, from, (size_t) (count * dev_size));
 		return;
 	}
 	const float* f = reinterpret_cast<const float*>(from);
@@ -61,13 +61,31 @@ void work(Job& j, int k)
 		if (e != cudaSuccess)
 			break;
 		const long long first = chunk * j.per_chunk;
-		deliver(j, j.c->pinned + (size_t) (2 * k + slot) * HostCopy::CHUNK, first, j.n - first < j.per_chunk ? j.n - first : j.per_chunk);
+		deliver(j.c->pinned + (size_t) (2 * k + slot) * HostCopy::CHUNK, j.dev_size, j.host, j.host_size, first,
+				j.n - first < j.per_chunk ? j.n - first : j.per_chunk);
 		slot ^= 1;
 	}
 	if (e != cudaSuccess) {
 		cudaStreamSynchronize(j.stream);  // nothing of ours is in flight into the pinned chunks
 		j.error = (int) e;
 	}
+}
+
+cudaError_t pageable_copy(cudaStream_t stream, const void* dev, int dev_size, void* host, int host_size, long long n)
+{
+	float chunk[4096];
+	const long long per_chunk = (long long) sizeof(chunk) / dev_size;
+	for (long long first = 0; first < n; first += per_chunk) {
+		const long long count = n - first < per_chunk ? n - first : per_chunk;
+		cudaError_t e = cudaMemcpyAsync(chunk, (const unsigned char*) dev + first * dev_size, (size_t) (count * dev_size),
+										cudaMemcpyDeviceToHost, stream);
+		if (e == cudaSuccess)
+			e = cudaStreamSynchronize(stream);
+		if (e != cudaSuccess)
+			return e;
+		deliver(reinterpret_cast<const unsigned char*>(chunk), dev_size, (unsigned char*) host, host_size, first, count);
+	}
+	return cudaSuccess;
 }
 
 }  // namespace
@@ -95,8 +113,10 @@ cudaError_t host_copy(HostCopy& c, int device, cudaStream_t stream, const void* 
 			if (e == cudaSuccess)
 				e = cudaEventCreateWithFlags(&ev, cudaEventDisableTiming);
 		if (e != cudaSuccess) {
+			// no pinned memory to be had: chunk by chunk through pageable memory
 			host_copy_free(c);
-			return e;
+			cudaGetLastError();
+			return pageable_copy(stream, dev, dev_size, host, host_size, n);
 		}
 	}
 	Job j;
