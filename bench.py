@@ -617,6 +617,10 @@ def run_adjoint(args):
     value = sites * steps * world / secs / 1e6
     v = lat.device_view()
     pop_bytes = v.sz * (spec["Z"] + 2) * v.elem_size  # all slots, ghost layer included
+    # the last steps' moments (16 B/site) are kept by the forward pass in the room a
+    # segment's populations would take (lbm_adjoint_forward), the others' recomputed
+    per_array = pop_bytes / (16 * sites)
+    recomputed = steps - max(0, min(int((every - 1) * per_array) - every, int(math.ceil(steps / every) * per_array), steps))
     lat.close()
     line = None
     if rank == 0:
@@ -628,19 +632,19 @@ def run_adjoint(args):
             "config": {"workload": spec["workload"], "lattice": [spec["X"], spec["Y"], spec["Z"]],
                        "samples": int(len(samples)), "checkpoint_every": every,
                        "checkpoint_memory_gb": round((math.ceil(steps / every) + every + 2) * pop_bytes / 1e9, 2)},
-            "gpu_launches": 3 * steps,
+            "gpu_launches": 2 * steps + recomputed,
             "forward_s": round(t_fwd, 4), "backward_s": round(t_bwd, 4), "objective": J,
             "grad_max_abs": float(np.max(np.abs(g[0]))),
             "roofline": {"bound": "hbm", "achieved": None, "peak": read_peaks()[0], "unit": "GB/s", "frac": None,
                          "traffic": None,
-                         "note": "per step: two primal A-A steps (216 B/site each), one adjoint step "
-                                 "(27 FP32 primal reads + 27 FP64 adjoint reads + 27 FP64 adjoint writes, 540 B/site) "
-                                 "and a 27-value FP32 copy per recomputed state (216 B/site)"},
+                         "note": "per step: a primal A-A step (216 B/site, 24 of force, 16 of moments), again for the "
+                                 "steps recomputed from a checkpoint, and one adjoint step (4 moments, 27 FP64 adjoint "
+                                 "values in and out, force, force gradient in and out: 520 B/site)"},
             "e2e": {"value": round(value, 2), "unit": "MLUPS", "h2d_bytes_per_step": 0, "d2h_bytes_per_step": 0,
                     "per_run": "lbm_adjoint_forward + lbm_adjoint_backward through the C-ABI"},
             "clocks": clk.summary(),
         }
-        bytes_per_site_step = 2 * 216 + 540 + 216
+        bytes_per_site_step = (216 + 24 + 16) * (1 + recomputed / steps) + 520
         line["roofline"]["achieved"] = round(bytes_per_site_step * sites * steps / secs / 1e9, 1)
         line["roofline"]["frac"] = round(line["roofline"]["achieved"] / line["roofline"]["peak"], 4)
     if dist is not None:
