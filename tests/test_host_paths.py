@@ -1,0 +1,92 @@
+"""Host paths that a healthy GPU does not reach -- memory that runs out, a launch
+that fails -- and the launches and copies that a call issues, on the CPU: the
+library over the runtime of fake_cudart.cpp, in a process of its own."""
+import os
+import subprocess
+import sys
+
+import pytest
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+CUDA = os.path.join(os.path.dirname(os.path.dirname(os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc"))), "include")
+
+PRELUDE = """
+import ctypes, os, sys
+import numpy as np
+import pytnl_lbm as pl
+lib = pl.library()
+fake = ctypes.CDLL(os.environ["FAKE_CUDART"])
+fake.fake_count.restype = ctypes.c_longlong
+fake.fake_trace.restype = ctypes.c_char_p
+fake.fake_in_use.restype = ctypes.c_size_t
+fake.fake_last_copy_to.restype = ctypes.c_void_p
+fake.fake_limit.argtypes = [ctypes.c_size_t]
+fake.fake_fail_launch.argtypes = fake.fake_fail_new.argtypes = [ctypes.c_longlong]
+fake.fake_pinned.argtypes = [ctypes.c_void_p, ctypes.c_size_t]
+def count(what): return fake.fake_count(what.encode())
+def refused(f, *a, **k):
+    try: f(*a, **k)
+    except pl.LbmError as e: return e.code
+    return 0
+"""
+
+
+@pytest.fixture(scope="module")
+def child(tmp_path_factory):
+    d = tmp_path_factory.mktemp("fake")
+    (d / "versions").write_text("libcudart.so.12 { global: *; };\n")
+    so = str(d / "libcudart.so.12")
+    subprocess.run(["g++", "-std=c++17", "-O1", "-shared", "-fPIC", "-I" + CUDA, "-Wl,-soname,libcudart.so.12",
+                    "-Wl,--version-script=" + str(d / "versions"), os.path.join(ROOT, "tests", "fake_cudart.cpp"),
+                    "-o", so], check=True)
+    env = dict(os.environ, LD_PRELOAD=so, FAKE_CUDART=so, PYTHONPATH=os.path.join(ROOT, "tnl-lbm_b200"))
+
+    def run(code):
+        r = subprocess.run([sys.executable, "-c", PRELUDE + code], capture_output=True, text=True, env=env, timeout=300)
+        assert r.returncode == 0, r.stdout + r.stderr
+    return run
+
+
+def test_step_over_the_fake_runtime(child):
+    """A step launches its kernel once, 16 steps go through a graph."""
+    child("""
+lat = pl.LBM(16, 8, 8, viscosity=0.01, periodic=True)
+fake.fake_reset()
+lat.step(3)
+assert count("launches") == 3, fake.fake_trace()
+lat.step(33)
+assert (count("nodes"), count("graph launches")) == (16, 2)
+assert lat.iteration == 36
+""")
+
+
+@pytest.mark.parametrize("room", ["checkpoints", "moments", "earlier moments", "all"])
+def test_adjoint_forward_falls_back_to_checkpoints(child, room):
+    """A forward pass runs wherever the checkpoints of all its steps and the
+    final state fit: without room for the kept moments (an earlier run holds the
+    checkpoints), with room for them but not for the checkpoints beside them, or
+    with the moments of an earlier run in the way of a run that keeps none."""
+    child("room = %r" % room + """
+N, K, X, Y, Z = 400, 20, 512, 8, 8
+lat = pl.LBM(X, Y, Z, viscosity=0.02, collision=pl.COLL_SRT, equilibrium=pl.EQ_SECOND_ORDER, periodic=True)
+v = lat.device_view()
+pop = v.sz * (Z + 2) * v.elem_size
+enough = fake.fake_in_use() + 24 * X * Y * Z + 48 + (N // K + 1) * pop
+def forward(n, every):
+    fake.fake_reset()
+    lat.adjoint_forward(np.zeros((3, Z, Y, X)), n, np.array([5]), np.zeros((1, 4)), checkpoint_every=every)
+if room == "checkpoints":
+    forward(N // K, 1)
+if room == "earlier moments":
+    forward(N, K)
+fake.fake_limit(0 if room == "all" else enough)
+n, every = (N // K, 1) if room == "earlier moments" else (N, K)
+forward(n, every)
+used = fake.fake_in_use()
+assert (used > enough) == (room == "all")  # the moments do not fit beside the checkpoints
+fake.fake_limit(0)
+lat.adjoint_backward()
+steps, recomputed = fake.fake_trace().count(b"adj_step_kernel"), fake.fake_trace().count(b"adj_primal_kernel") - n
+assert steps == n and (recomputed < n if room == "all" else recomputed == n), (steps, recomputed)
+lat.close()
+""")

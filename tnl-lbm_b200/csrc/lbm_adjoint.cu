@@ -12,8 +12,8 @@
 // segments from the last to the first: it restores the segment's checkpoint,
 // recomputes its steps and their moments in one working array, and runs the
 // adjoint steps backwards through them.  Peak memory is below (ceil(N/K) + K +
-// 2) population arrays, a forward pass alone takes at most 2 ceil(N/K) + 1;
-// K = sqrt(N) minimises it.
+// 2) population arrays, a forward pass alone takes up to 2 ceil(N/K) + 1 where
+// they fit and ceil(N/K) + 1 where they do not; K = sqrt(N) minimises it.
 //
 // On a 160x48x48 channel (FP32 primal, 64 steps, K = 8; B200) forward and
 // backward took 8.9 ms with the populations of a segment kept (a copy ahead of
@@ -368,16 +368,28 @@ int lbm_adjoint_forward(lbm_handle h, const double* force, int64_t nsteps, int64
 			return fail_free(afail(LBM_ERR_CUDA, "adjoint buffers: allocation failed"));
 		st->nsamples_cap = nsamples;
 	}
-	if (!ensure_bytes(st->kept_mom, st->kept_bytes, moments_bytes(h) * (size_t) kept))
-		kept = 0;  // no room: every step is recomputed
-	const long long nckpt = (nsteps - kept + every - 1) / every;
-	st->kept = kept;
-	while ((long long) st->ckpt.size() < nckpt) {
+	// the kept moments, then the checkpoints of the steps before them.  Where one
+	// or the other finds no room, nothing is kept (nor held from an earlier run)
+	// and every step is recomputed from the checkpoints alone.
+	long long nckpt = 0;
+	for (;;) {
+		if (!ensure_bytes(st->kept_mom, st->kept_bytes, moments_bytes(h) * (size_t) kept))
+			kept = 0;
+		nckpt = (nsteps - kept + every - 1) / every;
 		void* p = nullptr;
-		if (cudaMalloc(&p, h->pop_bytes) != cudaSuccess)
+		while ((long long) st->ckpt.size() < nckpt && cudaMalloc(&p, h->pop_bytes) == cudaSuccess)
+			st->ckpt.push_back(p);
+		if ((long long) st->ckpt.size() >= nckpt)
+			break;
+		if (!st->kept_mom)
 			return fail_free(afail(LBM_ERR_CUDA, "adjoint checkpoints: allocation of %lld x %zu bytes failed", nckpt, h->pop_bytes));
-		st->ckpt.push_back(p);
+		cudaGetLastError();
+		cudaFree(st->kept_mom);
+		st->kept_mom = nullptr;
+		st->kept_bytes = 0;
+		kept = 0;
 	}
+	st->kept = kept;
 	st->nckpt = nckpt;
 	if (cudaMemcpyAsync(st->force, force ? force : fh.data(), force_bytes, cudaMemcpyDefault, h->stream) != cudaSuccess
 		|| cudaMemcpyAsync(st->samples, samples, sizeof(long long) * nsamples, cudaMemcpyHostToDevice, h->stream) != cudaSuccess
