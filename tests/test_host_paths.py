@@ -90,3 +90,21 @@ steps, recomputed = fake.fake_trace().count(b"adj_step_kernel"), fake.fake_trace
 assert steps == n and (recomputed < n if room == "all" else recomputed == n), (steps, recomputed)
 lat.close()
 """)
+
+
+@pytest.mark.parametrize("shape", [(128, 0), (128, 1), (256, 3)])
+def test_ensemble_blocks_of_steps(child, shape):
+    """Several groups of members: a block of steps takes them one after the other,
+    a single step (also the odd one ahead of a block) all in one launch."""
+    child("shape = %r" % (shape,) + """
+ens = pl.Ensemble([(64, 32, 32)] * 30, [0.01] * 30, cum_flags=3)  # 212 MB
+ens.set_shape(*shape)
+for n, launches in ((1, 1), (1, 1), (3, 12), (1, 1)):
+    fake.fake_reset()
+    ens.step(n)
+    assert count("launches") == launches, (n, fake.fake_trace())
+fake.fake_reset()
+ens.step(1, sums=True)
+assert count("launches") == 2, fake.fake_trace()  # the step and the finish of the sums
+assert ens.iteration == 7
+""")

@@ -309,10 +309,12 @@ int ens_launch(lbm_ensemble e, int m0, int m1, long long iteration, bool sums, b
 }
 
 // n steps of every member from the parity of `iteration`, group by group (the
-// per-member launches of grid policy 2 need all members at once to fill the GPU)
+// per-member launches of grid policy 2 need all members at once to fill the GPU).
+// A single step finds no group in L2 and leaves none for a next one: one launch
+// over all members.
 int ens_block(lbm_ensemble e, long long iteration, long long n)
 {
-	if (e->grid_policy == 2) {
+	if (e->grid_policy == 2 || n == 1) {
 		for (long long s = 0; s < n; s++)
 			if (int rc = ens_launch(e, 0, e->count, iteration + s, false))
 				return rc;
