@@ -108,3 +108,18 @@ ens.step(1, sums=True)
 assert count("launches") == 2, fake.fake_trace()  # the step and the finish of the sums
 assert ens.iteration == 7
 """)
+
+
+def test_ensemble_graphs_are_bounded(child):
+    """A graph of 16 steps has a node per step and group: ensembles of up to 64
+    groups replay it, larger ones launch their (long) steps one by one."""
+    child("""
+for members, nodes, graph_launches, launches in ((30, 16 * 4, 2, 0), (620, 0, 0, 32 * 69)):
+    ens = pl.Ensemble([(64, 32, 32)] * members, [0.01] * members, cum_flags=3)  # 7.1 MB each
+    fake.fake_reset()
+    ens.step(32)
+    assert (count("nodes"), count("graph launches"), count("launches")) == (nodes, graph_launches, launches), \\
+        (count("nodes"), count("graph launches"), count("launches"))
+    assert ens.iteration == 32
+    ens.close()
+""")

@@ -81,6 +81,12 @@ __global__ void __launch_bounds__(256) ens_finish_kernel(const double* __restric
 struct lbm_ensemble_t
 {
 	static constexpr int GRAPH_STEPS = 16;
+	// Groups of members up to which their steps go into a graph.  Its nodes are
+	// GRAPH_STEPS a group and cost some 4 us each when it is built (first 50 steps
+	// after an autotune: 4 groups 0.5 ms more than later ones, 16 groups 1.0), while
+	// a group's step takes the GPU some 20 us, several times what its launch takes
+	// the host.
+	static constexpr int GRAPH_GROUPS = 64;
 
 	int count = 0;
 	int storage = 0, collision = 0, cum_flags = 0, equilibrium = 0, device = 0, use_graphs = 1;
@@ -358,7 +364,8 @@ int ens_plain_steps(lbm_ensemble e, long long n)
 {
 	// to an even step ahead of a graph; a block of steps that no graph follows
 	// runs as one
-	const bool graphs = e->use_graphs && n - e->iteration % 2 >= lbm_ensemble_t::GRAPH_STEPS;
+	const bool graphs = e->use_graphs && n - e->iteration % 2 >= lbm_ensemble_t::GRAPH_STEPS
+					 && (e->grid_policy == 2 || (int) e->group0.size() - 1 <= lbm_ensemble_t::GRAPH_GROUPS);
 	if (graphs && e->iteration % 2 != 0) {
 		if (int rc = ens_block(e, e->iteration, 1))
 			return rc;
