@@ -123,3 +123,22 @@ for members, nodes, graph_launches, launches in ((30, 16 * 4, 2, 0), (620, 0, 0,
     assert ens.iteration == 32
     ens.close()
 """)
+
+
+@pytest.mark.parametrize("kind", ["lattice", "ensemble"])
+def test_failed_launch_is_reported_once(child, kind):
+    """The error of a step launch is that call's; the next call does not find it
+    in the runtime and report it as its own."""
+    child("kind = %r" % kind + """
+if kind == "lattice":
+    sim = pl.LBM(16, 8, 8, viscosity=0.01, periodic=True)
+    read = sim.get_populations
+else:
+    sim = pl.Ensemble([(16, 8, 8)] * 2, [0.01] * 2)
+    read = lambda: sim.get_populations(1)
+fake.fake_fail_launch(1)
+assert refused(sim.step, 1) == 3 and sim.iteration == 0
+read()
+sim.step(1)
+assert sim.iteration == 1
+""")

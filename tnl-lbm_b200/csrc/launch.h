@@ -15,7 +15,9 @@ namespace lbm {
 // copy, a wait on an event) it starts as an ordinary launch.  Only for kernels
 // whose every thread begins with await_predecessor: one that did not wait could
 // complete, and let its own dependents go, ahead of its predecessor.
-// dependent = false: an ordinary launch.
+// dependent = false: an ordinary launch.  The error of a launch that fails is
+// taken from the runtime, as cudaGetLastError after <<<>>> does: left there, the
+// next launch to ask for it would report it as its own.
 template <typename... P, typename... A>
 inline cudaError_t launch_dependent(bool dependent, void (*kernel)(P...), dim3 grid, dim3 block, cudaStream_t stream, A... args)
 {
@@ -28,9 +30,11 @@ inline cudaError_t launch_dependent(bool dependent, void (*kernel)(P...), dim3 g
 	cfg.stream = stream;
 	cfg.attrs = &attr;
 	cfg.numAttrs = dependent ? 1 : 0;
-	return cudaLaunchKernelEx(&cfg, kernel, P(args)...);
+	const cudaError_t err = cudaLaunchKernelEx(&cfg, kernel, P(args)...);
+	if (err != cudaSuccess)
+		cudaGetLastError();
+	return err;
 }
-
 
 enum Storage : int
 {
