@@ -333,7 +333,9 @@ LBM_API int lbm_ensemble_init_equilibrium(lbm_ensemble e, double rho0, double vx
 LBM_API int lbm_ensemble_set_populations(lbm_ensemble e, int member, const void* host, int layout, int dtype);
 LBM_API int lbm_ensemble_get_populations(lbm_ensemble e, int member, void* host, int layout, int dtype);
 /* nsteps A-A steps of every member; LBM_STEP_SUMS computes per-member sums
- * in the last step (lbm_ensemble_get_sums). */
+ * in the last step (lbm_ensemble_get_sums).  When a launch fails part way the
+ * members may be left at different steps: steps and read-out are then refused
+ * (LBM_ERR_INVALID) until lbm_ensemble_init_*. */
 LBM_API int lbm_ensemble_step(lbm_ensemble e, int64_t nsteps, int flags);
 /* out[count][6]: the sums of lbm_get_sums for each member */
 LBM_API int lbm_ensemble_get_sums(lbm_ensemble e, double* out);

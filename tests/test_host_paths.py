@@ -142,3 +142,36 @@ read()
 sim.step(1)
 assert sim.iteration == 1
 """)
+
+
+@pytest.mark.parametrize("graphs", [0, 1])
+@pytest.mark.parametrize("shape", [(128, 0), (256, 3)])
+def test_failed_launch_leaves_no_members_apart(child, shape, graphs):
+    """A block of steps whose launch fails part way has some groups ahead of the
+    others: the ensemble refuses steps and read-out until it is initialised.  A
+    launch that fails before any went out (or under capture) changes nothing."""
+    child("shape, graphs = %r, %r" % (shape, graphs) + """
+ens = pl.Ensemble([(64, 32, 32)] * 30, [0.01] * 30, cum_flags=3, use_graphs=graphs)  # 4 groups
+ens.set_shape(*shape)
+ens.init_taylor_green(0.05)
+ens.step(2)
+for n in (1, 3):
+    fake.fake_fail_launch(1)
+    assert refused(ens.step, n) == 3 and ens.iteration == 2
+if graphs:
+    fake.fake_fail_launch(9)
+    assert refused(ens.step, 16) == 3 and ens.iteration == 2
+    ens.step(16)
+else:
+    ens.step(16)
+ens.get_populations(0)
+fake.fake_fail_launch(6)
+assert refused(ens.step, 3) == 3
+for call in (lambda: ens.step(1), lambda: ens.step(3), ens.autotune, lambda: ens.get_populations(0)):
+    assert refused(call) == 1
+    assert "part way" in lib.lbm_last_error().decode()
+ens.init_taylor_green(0.05)
+ens.step(3)
+ens.get_populations(29)
+assert ens.iteration == 3
+""")

@@ -108,6 +108,7 @@ struct lbm_ensemble_t
 	double* sums_host = nullptr;	 // pinned [count][NRED]
 	double* sums_mapped = nullptr;	 // device address of sums_host
 	bool sums_valid = false;
+	bool torn = false;	// a block of steps failed part way: members are at different steps
 	long long iteration = 0;
 	cudaGraphExec_t graph = nullptr;
 	lbm::HostCopy host_copy;  // staging of the populations handed to the caller
@@ -157,6 +158,16 @@ int echeck(lbm_ensemble e)
 		return efail(LBM_ERR_INVALID, "null ensemble handle");
 	if (cudaSetDevice(e->device) != cudaSuccess)
 		return efail(LBM_ERR_CUDA, "cudaSetDevice(%d) failed", e->device);
+	return LBM_OK;
+}
+
+// echeck, and that the members are all at the step of e->iteration
+int echeck_state(lbm_ensemble e)
+{
+	if (int rc = echeck(e))
+		return rc;
+	if (e->torn)
+		return efail(LBM_ERR_INVALID, "a block of steps failed part way and left members at different steps: initialise again");
 	return LBM_OK;
 }
 
@@ -317,20 +328,36 @@ int ens_launch(lbm_ensemble e, int m0, int m1, long long iteration, bool sums, b
 // n steps of every member from the parity of `iteration`, group by group (the
 // per-member launches of grid policy 2 need all members at once to fill the GPU).
 // A single step finds no group in L2 and leaves none for a next one: one launch
-// over all members.
-int ens_block(lbm_ensemble e, long long iteration, long long n)
+// over all members.  launched: steps launched, of whatever members.
+int ens_block(lbm_ensemble e, long long iteration, long long n, long long& launched)
 {
+	launched = 0;
 	if (e->grid_policy == 2 || n == 1) {
-		for (long long s = 0; s < n; s++)
+		for (long long s = 0; s < n; s++, launched++)
 			if (int rc = ens_launch(e, 0, e->count, iteration + s, false))
 				return rc;
 		return LBM_OK;
 	}
 	for (size_t k = 0; k + 1 < e->group0.size(); k++)
-		for (long long s = 0; s < n; s++)
+		for (long long s = 0; s < n; s++, launched++)
 			if (int rc = ens_launch(e, e->group0[k], e->group0[k + 1], iteration + s, false))
 				return rc;
 	return LBM_OK;
+}
+
+// the same from e->iteration, which moves on by the steps that all members took;
+// a failure that leaves them apart is marked
+int ens_advance(lbm_ensemble e, long long n)
+{
+	long long launched;
+	const int rc = ens_block(e, e->iteration, n, launched);
+	if (rc == LBM_OK)
+		e->iteration += n;
+	else if (e->grid_policy == 2)
+		e->iteration += launched;
+	else if (launched > 0)
+		e->torn = true;
+	return rc;
 }
 
 int ens_build_graph(lbm_ensemble e)
@@ -342,7 +369,8 @@ int ens_build_graph(lbm_ensemble e)
 			return rc;
 	cudaGraph_t graph = nullptr;
 	ENS_CUDA(cudaStreamBeginCapture(e->stream, cudaStreamCaptureModeThreadLocal));
-	const int rc = ens_block(e, 0, lbm_ensemble_t::GRAPH_STEPS);  // the graph starts at an even step
+	long long launched;
+	const int rc = ens_block(e, 0, lbm_ensemble_t::GRAPH_STEPS, launched);  // the graph starts at an even step
 	const cudaError_t end = cudaStreamEndCapture(e->stream, &graph);
 	if (rc != LBM_OK) {
 		if (graph)
@@ -367,9 +395,8 @@ int ens_plain_steps(lbm_ensemble e, long long n)
 	const bool graphs = e->use_graphs && n - e->iteration % 2 >= lbm_ensemble_t::GRAPH_STEPS
 					 && (e->grid_policy == 2 || (int) e->group0.size() - 1 <= lbm_ensemble_t::GRAPH_GROUPS);
 	if (graphs && e->iteration % 2 != 0) {
-		if (int rc = ens_block(e, e->iteration, 1))
+		if (int rc = ens_advance(e, 1))
 			return rc;
-		e->iteration++;
 		n--;
 	}
 	if (graphs && n >= lbm_ensemble_t::GRAPH_STEPS) {
@@ -382,10 +409,7 @@ int ens_plain_steps(lbm_ensemble e, long long n)
 			n -= lbm_ensemble_t::GRAPH_STEPS;
 		}
 	}
-	if (int rc = ens_block(e, e->iteration, n))
-		return rc;
-	e->iteration += n;
-	return LBM_OK;
+	return ens_advance(e, n);
 }
 
 size_t dense_count(const lbm::Geometry& g, int layout)
@@ -403,6 +427,7 @@ int ens_init(lbm_ensemble e, const lbm::InitSpec& spec)
 	}
 	e->iteration = 0;
 	e->sums_valid = false;
+	e->torn = false;
 	ENS_CUDA(cudaStreamSynchronize(e->stream));
 	return LBM_OK;
 }
@@ -567,7 +592,7 @@ int lbm_ensemble_set_populations(lbm_ensemble e, int member, const void* host, i
 
 int lbm_ensemble_get_populations(lbm_ensemble e, int member, void* host, int layout, int dtype)
 {
-	if (int rc = echeck(e))
+	if (int rc = echeck_state(e))
 		return rc;
 	if (member < 0 || member >= e->count)
 		return efail(LBM_ERR_INVALID, "member %d out of range", member);
@@ -591,7 +616,7 @@ int lbm_ensemble_get_populations(lbm_ensemble e, int member, void* host, int lay
 
 int lbm_ensemble_step(lbm_ensemble e, int64_t nsteps, int flags)
 {
-	if (int rc = echeck(e))
+	if (int rc = echeck_state(e))
 		return rc;
 	if (nsteps < 0 || (nsteps == 0 && flags))
 		return efail(LBM_ERR_INVALID, "nsteps must be positive when flags are given");
@@ -682,7 +707,7 @@ int lbm_ensemble_get_shape(lbm_ensemble e, int* tile_sites, int* grid_policy)
 
 int lbm_ensemble_autotune(lbm_ensemble e, int ntrials)
 {
-	if (int rc = echeck(e))
+	if (int rc = echeck_state(e))
 		return rc;
 	if (ntrials < 1)
 		return efail(LBM_ERR_INVALID, "ntrials must be positive");
@@ -731,6 +756,7 @@ int lbm_ensemble_autotune(lbm_ensemble e, int ntrials)
 	cudaMemcpyAsync(e->pops, backup, e->pop_bytes, cudaMemcpyDeviceToDevice, e->stream);
 	cudaStreamSynchronize(e->stream);
 	cudaFree(backup);
+	e->torn = false;
 	if (rc)
 		return rc;
 	const cudaError_t err = cudaGetLastError();
