@@ -175,3 +175,33 @@ ens.step(3)
 ens.get_populations(29)
 assert ens.iteration == 3
 """)
+
+
+FIELD = """
+def field(storage, X, Y, Z):
+    # a lattice whose macro field in device memory holds numbers of its own
+    lat = pl.LBM(X, Y, Z, viscosity=0.01, periodic=True, storage=getattr(pl, "STORE_" + storage))
+    lat.step(1, macro=True)
+    n, t = 4 * X * Y * Z, np.float64 if storage == "F64" else np.float32
+    a = np.random.default_rng(1).standard_normal(n).astype(t)
+    ctypes.memmove(lat.device_view().macro, a.ctypes.data, a.nbytes)
+    fake.fake_reset()
+    return lat, a.astype(np.float64)
+def read(lat, out):
+    assert lib.lbm_get_macro(lat.h, out.ctypes.data_as(ctypes.POINTER(ctypes.c_double))) == 0
+"""
+
+
+@pytest.mark.parametrize("storage,direct", [("F64", True), ("F32", False)])
+def test_field_copy_into_pinned_memory_is_direct(child, storage, direct):
+    """Pinned memory of the caller takes the field in one copy of the device where
+    the values go as they are; values to be widened are staged."""
+    child(FIELD + "storage, direct = %r, %r" % (storage, direct) + """
+lat, want = field(storage, 64, 64, 64)
+out = np.zeros_like(want)
+fake.fake_pinned(out.ctypes.data, out.nbytes)
+read(lat, out)
+np.testing.assert_array_equal(out, want)
+assert (fake.fake_last_copy_to() == out.ctypes.data, count("pinned allocations")) == (direct, 0 if direct else 1)
+assert not direct or count("copies to the host") == 1
+""")

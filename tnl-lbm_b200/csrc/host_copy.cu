@@ -1,4 +1,4 @@
-// Device-to-host copies of fields into pageable memory (host_copy.h).
+// Device-to-host copies of fields into the caller's memory (host_copy.h).
 #include "host_copy.h"
 
 #include <atomic>
@@ -71,6 +71,17 @@ void work(Job& j, int k)
 	}
 }
 
+// memory that the runtime knows (pinned, registered, managed): the device copies into it itself
+bool reached_by_device(const void* host)
+{
+	cudaPointerAttributes a;
+	if (cudaPointerGetAttributes(&a, host) != cudaSuccess) {
+		cudaGetLastError();
+		return false;
+	}
+	return a.type != cudaMemoryTypeUnregistered;
+}
+
 cudaError_t pageable_copy(cudaStream_t stream, const void* dev, int dev_size, void* host, int host_size, long long n)
 {
 	float chunk[4096];
@@ -107,6 +118,10 @@ cudaError_t host_copy(HostCopy& c, int device, cudaStream_t stream, const void* 
 {
 	if (n < 1)
 		return cudaStreamSynchronize(stream);
+	if (dev_size == host_size && reached_by_device(host)) {
+		const cudaError_t e = cudaMemcpyAsync(host, dev, (size_t) n * dev_size, cudaMemcpyDeviceToHost, stream);
+		return e == cudaSuccess ? cudaStreamSynchronize(stream) : e;
+	}
 	if (!c.pinned) {
 		cudaError_t e = cudaMallocHost((void**) &c.pinned, 2 * HostCopy::THREADS * HostCopy::CHUNK);
 		for (cudaEvent_t& ev : c.landed)
