@@ -205,3 +205,17 @@ np.testing.assert_array_equal(out, want)
 assert (fake.fake_last_copy_to() == out.ctypes.data, count("pinned allocations")) == (direct, 0 if direct else 1)
 assert not direct or count("copies to the host") == 1
 """)
+
+
+@pytest.mark.parametrize("storage,shape,copies", [("F64", (64, 64, 65), 1), ("F32", (64, 64, 65), 2), ("F32", (8, 4, 4), 1)])
+def test_field_copy_without_pinned_memory(child, storage, shape, copies):
+    """No pinned memory to be had: one pageable copy of values that go as they
+    are, chunks of a million values where they are widened."""
+    child(FIELD + "storage, shape, copies = %r, %r, %r" % (storage, shape, copies) + """
+lat, want = field(storage, *shape)
+fake.fake_no_pinned(1)
+out = np.zeros_like(want)
+read(lat, out)
+np.testing.assert_array_equal(out, want)
+assert count("copies to the host") == copies, count("copies to the host")
+""")

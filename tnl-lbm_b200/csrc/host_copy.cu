@@ -4,6 +4,8 @@
 #include <atomic>
 #include <cstring>
 #include <functional>
+#include <memory>
+#include <new>
 #include <system_error>
 #include <thread>
 
@@ -82,14 +84,26 @@ bool reached_by_device(const void* host)
 	return a.type != cudaMemoryTypeUnregistered;
 }
 
+cudaError_t direct_copy(cudaStream_t stream, const void* dev, void* host, size_t bytes)
+{
+	const cudaError_t e = cudaMemcpyAsync(host, dev, bytes, cudaMemcpyDeviceToHost, stream);
+	return e == cudaSuccess ? cudaStreamSynchronize(stream) : e;
+}
+
+// without pinned memory: one copy where the values go as they are, else through
+// a buffer of as many values as there is memory for
 cudaError_t pageable_copy(cudaStream_t stream, const void* dev, int dev_size, void* host, int host_size, long long n)
 {
-	float chunk[4096];
-	const long long per_chunk = (long long) sizeof(chunk) / dev_size;
+	if (dev_size == host_size)
+		return direct_copy(stream, dev, host, (size_t) n * dev_size);
+	float small[4096];
+	const long long many = n < (1 << 20) ? n : 1 << 20;
+	std::unique_ptr<float[]> large(new (std::nothrow) float[(size_t) many]);
+	float* const chunk = large ? large.get() : small;
+	const long long per_chunk = large ? many : 4096;
 	for (long long first = 0; first < n; first += per_chunk) {
 		const long long count = n - first < per_chunk ? n - first : per_chunk;
-		cudaError_t e = cudaMemcpyAsync(chunk, (const unsigned char*) dev + first * dev_size, (size_t) (count * dev_size),
-										cudaMemcpyDeviceToHost, stream);
+		cudaError_t e = cudaMemcpyAsync(chunk, (const float*) dev + first, (size_t) count * sizeof(float), cudaMemcpyDeviceToHost, stream);
 		if (e == cudaSuccess)
 			e = cudaStreamSynchronize(stream);
 		if (e != cudaSuccess)
@@ -118,17 +132,15 @@ cudaError_t host_copy(HostCopy& c, int device, cudaStream_t stream, const void* 
 {
 	if (n < 1)
 		return cudaStreamSynchronize(stream);
-	if (dev_size == host_size && reached_by_device(host)) {
-		const cudaError_t e = cudaMemcpyAsync(host, dev, (size_t) n * dev_size, cudaMemcpyDeviceToHost, stream);
-		return e == cudaSuccess ? cudaStreamSynchronize(stream) : e;
-	}
+	if (dev_size == host_size && reached_by_device(host))
+		return direct_copy(stream, dev, host, (size_t) n * dev_size);
 	if (!c.pinned) {
 		cudaError_t e = cudaMallocHost((void**) &c.pinned, 2 * HostCopy::THREADS * HostCopy::CHUNK);
 		for (cudaEvent_t& ev : c.landed)
 			if (e == cudaSuccess)
 				e = cudaEventCreateWithFlags(&ev, cudaEventDisableTiming);
 		if (e != cudaSuccess) {
-			// no pinned memory to be had: chunk by chunk through pageable memory
+			// no pinned memory to be had
 			host_copy_free(c);
 			cudaGetLastError();
 			return pageable_copy(stream, dev, dev_size, host, host_size, n);
