@@ -19,8 +19,8 @@ std::map<const void*, std::string> kernel_names;
 std::map<std::string, long long> counts;
 std::string trace;	// kernels launched since fake_reset, one a line
 size_t in_use = 0, limit = 0;
-long long launch_to_fail = 0;
-bool no_pinned = false, arm_new = false;
+long long launch_to_fail = 0, news_armed = 0;
+bool no_pinned = false;
 const char *pinned_first = nullptr, *pinned_last = nullptr;
 const void* last_copy_to = nullptr;
 thread_local cudaError_t last_error = cudaSuccess;
@@ -58,8 +58,10 @@ cudaError_t launch(const void* func)
 
 void* operator new(size_t n)
 {
-	if (news_left > 0 && --news_left == 0)
+	if (news_left > 0 && --news_left == 0) {
+		counts["thrown"]++;
 		throw std::bad_alloc();
+	}
 	if (void* p = std::malloc(n ? n : 1))
 		return p;
 	throw std::bad_alloc();
@@ -113,11 +115,12 @@ const void* fake_last_copy_to()
 {
 	return last_copy_to;
 }
-// the n-th operator new of the thread after its next synchronisation throws
+// the n-th operator new of the thread after its next synchronisation throws (the
+// names of counts are short and there already: this file allocates nothing there)
 void fake_fail_new(long long n)
 {
-	arm_new = n > 0;
-	counts["arm"] = n;
+	counts["host copies"] = counts["thrown"] = 0;
+	news_armed = n;
 }
 
 void** __cudaRegisterFatBinary(void*)
@@ -230,7 +233,7 @@ cudaError_t cudaMalloc(void** p, size_t n)
 		return give(cudaErrorMemoryAllocation);
 	device_memory[*p] = n;
 	in_use += n;
-	counts["device allocations"]++;
+	counts["allocations"]++;
 	return cudaSuccess;
 }
 cudaError_t cudaFree(void* p)
@@ -258,7 +261,7 @@ cudaError_t cudaMallocHost(void** p, size_t n)
 	if (no_pinned)
 		return give(cudaErrorMemoryAllocation);
 	*p = std::calloc(n, 1);
-	counts["pinned allocations"]++;
+	counts["pinned"]++;
 	return cudaSuccess;
 }
 cudaError_t cudaHostAlloc(void** p, size_t n, unsigned)
@@ -287,7 +290,7 @@ cudaError_t cudaMemcpyAsync(void* to, const void* from, size_t n, cudaMemcpyKind
 	std::memcpy(to, from, n);
 	std::lock_guard<std::mutex> lock(mutex);
 	if (kind == cudaMemcpyDeviceToHost) {
-		counts["copies to the host"]++;
+		counts["host copies"]++;
 		last_copy_to = to;
 	}
 	return cudaSuccess;
@@ -313,9 +316,9 @@ cudaError_t cudaStreamDestroy(cudaStream_t s)
 }
 cudaError_t cudaStreamSynchronize(cudaStream_t)
 {
-	if (arm_new) {
-		arm_new = false;
-		news_left = counts["arm"];
+	if (news_armed > 0) {
+		news_left = news_armed;
+		news_armed = 0;
 	}
 	return cudaSuccess;
 }

@@ -34,7 +34,7 @@ def refused(f, *a, **k):
 @pytest.fixture(scope="module")
 def child(tmp_path_factory):
     d = tmp_path_factory.mktemp("fake")
-    (d / "versions").write_text("libcudart.so.12 { global: *; };\n")
+    (d / "versions").write_text("libcudart.so.12 { global: cuda*; __cuda*; fake_*; };\n")
     so = str(d / "libcudart.so.12")
     subprocess.run(["g++", "-std=c++17", "-O1", "-shared", "-fPIC", "-I" + CUDA, "-Wl,-soname,libcudart.so.12",
                     "-Wl,--version-script=" + str(d / "versions"), os.path.join(ROOT, "tests", "fake_cudart.cpp"),
@@ -202,8 +202,8 @@ out = np.zeros_like(want)
 fake.fake_pinned(out.ctypes.data, out.nbytes)
 read(lat, out)
 np.testing.assert_array_equal(out, want)
-assert (fake.fake_last_copy_to() == out.ctypes.data, count("pinned allocations")) == (direct, 0 if direct else 1)
-assert not direct or count("copies to the host") == 1
+assert (fake.fake_last_copy_to() == out.ctypes.data, count("pinned")) == (direct, 0 if direct else 1)
+assert not direct or count("host copies") == 1
 """)
 
 
@@ -217,5 +217,18 @@ fake.fake_no_pinned(1)
 out = np.zeros_like(want)
 read(lat, out)
 np.testing.assert_array_equal(out, want)
-assert count("copies to the host") == copies, count("copies to the host")
+assert count("host copies") == copies, count("host copies")
+""")
+
+
+@pytest.mark.parametrize("which", [1, 2, 3])
+def test_field_copy_without_memory_for_a_thread(child, which):
+    """No memory for the state of a helper thread: the caller takes its share."""
+    child(FIELD + "which = %r" % which + """
+lat, want = field("F32", 64, 64, 64)  # 16 chunks: four threads
+out = np.zeros_like(want)
+fake.fake_fail_new(which)
+read(lat, out)
+np.testing.assert_array_equal(out, want)
+assert count("thrown") == 1
 """)

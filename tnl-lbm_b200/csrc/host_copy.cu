@@ -3,10 +3,10 @@
 
 #include <atomic>
 #include <cstring>
+#include <exception>
 #include <functional>
 #include <memory>
 #include <new>
-#include <system_error>
 #include <thread>
 
 namespace lbm {
@@ -170,8 +170,9 @@ cudaError_t host_copy(HostCopy& c, int device, cudaStream_t stream, const void* 
 			for (; started < HostCopy::THREADS - 1; started++)
 				helpers[started] = std::thread(work, std::ref(j), started + 1);
 		}
-		catch (const std::system_error&) {
-			// no more threads to be had: this one takes the others' shares below
+		catch (const std::exception&) {
+			// no more threads to be had, or no memory for one: this one takes the
+			// others' shares below
 		}
 	}
 	for (int k = 0; k < j.threads; k++)
