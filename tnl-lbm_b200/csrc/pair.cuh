@@ -343,13 +343,14 @@ struct PairAt
 	// ragged rows only: x offset of the first site's right neighbour, 1 or the
 	// wrap of a pair whose second site lies past the row's end
 	int mid;
+	int last;	  // ragged rows only: x offset of the second site's left neighbour from the first site
 	bool single;  // ragged rows only: the pair's second site lies past the row's end
 };
 
 // neighbours of the pair (x, x + 1) of row (y, z) of the population array f
 // (element size E bytes, strides in elements): periodic sites wrap in x and
 // y (wrap) and in z (wrap && zwrap), all others reach the ghost layer
-__device__ __forceinline__ PairAt pair_at_of(char* f, long long E, int sy, int sz, int x0, int X, int Y, int Z, int x, int y,
+__host__ __device__ __forceinline__ PairAt pair_at_of(char* f, long long E, int sy, int sz, int x0, int X, int Y, int Z, int x, int y,
 											 int z, bool wrap, bool zwrap)
 {
 	PairAt at;
@@ -365,20 +366,31 @@ __device__ __forceinline__ PairAt pair_at_of(char* f, long long E, int sy, int s
 	at.left = (wrap && x == 0) ? X - 1 : -1;
 	at.right = (wrap && x + 1 == X - 1) ? -(X - 1) : 1;
 	at.mid = 1;
+	at.last = 0;
 	at.single = false;
 	return at;
 }
 
 // The last pair of a periodic row of odd width has one site (x = X - 1): its
-// second lane reads within the row (the ghost site x = X, or what the first
-// lane reads), computes along and is never stored.
-__device__ __forceinline__ void pair_ragged(PairAt& at, int x, int X)
+// second lane reads what no other thread writes (the ghost site x = X, or what
+// the first lane reads), computes along and is never stored.
+__host__ __device__ __forceinline__ void pair_ragged(PairAt& at, int x, int X)
 {
 	if (x + 1 == X) {
 		at.single = true;
 		at.mid = -(X - 1);
 		at.right = 0;
+		at.last = at.left;
 	}
+}
+
+// x offsets, from the pair's first site, of what its two lanes read of a
+// direction with x component CX in an odd step
+template <int CX>
+__host__ __device__ __forceinline__ void pair_lanes(const PairAt& at, int& first, int& second)
+{
+	first = CX > 0 ? at.left : CX < 0 ? at.mid : 0;
+	second = CX > 0 ? at.last : CX < 0 ? at.mid + at.right : 1;
 }
 
 template <typename T>
@@ -405,10 +417,13 @@ __device__ __forceinline__ void pair_read_at(const PairAt& at, const PairSlots& 
 				const T* c = reinterpret_cast<const T*>(at.P[1 - cz(q)] + at.oy[1 - cy(q)] + ps.b[opp(q)]);
 				if constexpr (cx(q) == 0)
 					s.f[q] = IO::template load2<opp(q)>(c);
+				else if constexpr (RAGGED) {
+					int first, second;
+					pair_lanes<cx(q)>(at, first, second);
+					s.f[q] = F2(S::template load<opp(q)>(c + first), S::template load<opp(q)>(c + second));
+				}
 				else if constexpr (cx(q) > 0)
 					s.f[q] = F2(S::template load<opp(q)>(c + at.left), S::template load<opp(q)>(c));
-				else if constexpr (RAGGED)
-					s.f[q] = F2(S::template load<opp(q)>(c + at.mid), S::template load<opp(q)>(c + at.mid + at.right));
 				else
 					s.f[q] = F2(S::template load<opp(q)>(c + 1), S::template load<opp(q)>(c + 1 + at.right));
 			}
