@@ -577,6 +577,16 @@ def tgv512_throughput(pl, device, steps, warmup, kernel16="pair"):
     return out
 
 
+def adjoint_traffic(steps, every, pop_bytes, sites):
+    """(steps recomputed in the backward pass, bytes per site and step) of an FP32
+    gradient.  The last steps' moments (16 B/site) are kept by the forward pass in
+    the room a segment's populations would take (lbm_adjoint_forward, with memory
+    for them), the others' are written when their steps are recomputed."""
+    per_array = pop_bytes / (16 * sites)
+    recomputed = steps - max(0, min(int((every - 1) * per_array) - every, int(math.ceil(steps / every) * per_array), steps))
+    return recomputed, (216 + 24) * (1 + recomputed / steps) + 16 + 520
+
+
 def run_adjoint(args):
     """Forward pass with checkpoints plus backward pass of the discrete adjoint;
     value = sites x steps / (forward + backward device time)."""
@@ -617,10 +627,7 @@ def run_adjoint(args):
     value = sites * steps * world / secs / 1e6
     v = lat.device_view()
     pop_bytes = v.sz * (spec["Z"] + 2) * v.elem_size  # all slots, ghost layer included
-    # the last steps' moments (16 B/site) are kept by the forward pass in the room a
-    # segment's populations would take (lbm_adjoint_forward), the others' recomputed
-    per_array = pop_bytes / (16 * sites)
-    recomputed = steps - max(0, min(int((every - 1) * per_array) - every, int(math.ceil(steps / every) * per_array), steps))
+    recomputed, bytes_per_site_step = adjoint_traffic(steps, every, pop_bytes, sites)
     lat.close()
     line = None
     if rank == 0:
@@ -637,14 +644,13 @@ def run_adjoint(args):
             "grad_max_abs": float(np.max(np.abs(g[0]))),
             "roofline": {"bound": "hbm", "achieved": None, "peak": read_peaks()[0], "unit": "GB/s", "frac": None,
                          "traffic": None,
-                         "note": "per step: a primal A-A step (216 B/site, 24 of force, 16 of moments), again for the "
-                                 "steps recomputed from a checkpoint, and one adjoint step (4 moments, 27 FP64 adjoint "
-                                 "values in and out, force, force gradient in and out: 520 B/site)"},
+                         "note": "per step: a primal A-A step (216 B/site, 24 of force), again for the steps recomputed "
+                                 "from a checkpoint, its moments written once (16), and one adjoint step (4 moments, 27 "
+                                 "FP64 adjoint values in and out, force, force gradient in and out: 520 B/site)"},
             "e2e": {"value": round(value, 2), "unit": "MLUPS", "h2d_bytes_per_step": 0, "d2h_bytes_per_step": 0,
                     "per_run": "lbm_adjoint_forward + lbm_adjoint_backward through the C-ABI"},
             "clocks": clk.summary(),
         }
-        bytes_per_site_step = (216 + 24 + 16) * (1 + recomputed / steps) + 520
         line["roofline"]["achieved"] = round(bytes_per_site_step * sites * steps / secs / 1e9, 1)
         line["roofline"]["frac"] = round(line["roofline"]["achieved"] / line["roofline"]["peak"], 4)
     if dist is not None:

@@ -232,3 +232,23 @@ read(lat, out)
 np.testing.assert_array_equal(out, want)
 assert count("thrown") == 1
 """)
+
+
+@pytest.mark.parametrize("steps,every", [(64, 8), (400, 20), (100, 50), (9, 1)])
+def test_bench_counts_the_adjoint_steps_that_run(child, steps, every):
+    """The bench's traffic of a gradient: every primal step that runs moves its
+    populations and force, every step's moments are written once."""
+    child("steps, every = %d, %d" % (steps, every) + """
+sys.path.insert(0, %r)""" % ROOT + """
+import bench
+X, Y, Z = 512, 8, 8
+lat = pl.LBM(X, Y, Z, viscosity=0.02, collision=pl.COLL_SRT, equilibrium=pl.EQ_SECOND_ORDER, periodic=True)
+v = lat.device_view()
+fake.fake_reset()
+lat.adjoint_forward(np.zeros((3, Z, Y, X)), steps, np.array([5]), np.zeros((1, 4)), checkpoint_every=every)
+lat.adjoint_backward()
+primal = fake.fake_trace().count(b"adj_primal_kernel")
+recomputed, site_bytes = bench.adjoint_traffic(steps, every, v.sz * (Z + 2) * v.elem_size, X * Y * Z)
+assert recomputed == primal - steps
+assert abs(site_bytes - (240 * primal / steps + 16 + 520)) < 1e-9, site_bytes
+""")
