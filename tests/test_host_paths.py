@@ -192,32 +192,52 @@ def read(lat, out):
 """
 
 
-@pytest.mark.parametrize("storage,direct", [("F64", True), ("F32", False)])
-def test_field_copy_into_pinned_memory_is_direct(child, storage, direct):
-    """Pinned memory of the caller takes the field in one copy of the device where
-    the values go as they are; values to be widened are staged."""
-    child(FIELD + "storage, direct = %r, %r" % (storage, direct) + """
-lat, want = field(storage, 64, 64, 64)
-out = np.zeros_like(want)
-fake.fake_pinned(out.ctypes.data, out.nbytes)
-read(lat, out)
-np.testing.assert_array_equal(out, want)
-assert (fake.fake_last_copy_to() == out.ctypes.data, count("pinned")) == (direct, 0 if direct else 1)
-assert not direct or count("host copies") == 1
+@pytest.mark.parametrize("storage", ["F64", "F32"])
+def test_field_copies_of_a_new_lattice(child, storage):
+    """The first read-outs of a lattice pay for no staging: values that go as they
+    are take one copy below 32 MB, values to be widened are copied into the
+    caller's memory and widened there, until 4 MB have gone that way."""
+    child(FIELD + "storage = %r" % storage + """
+lat, want = field(storage, 33, 32, 31)  # 1 MB
+for k in range(20):
+    out = np.zeros_like(want)
+    fake.fake_reset()
+    read(lat, out)
+    np.testing.assert_array_equal(out, want)
+    if storage == "F32" and (k + 1) * out.nbytes >= 4 << 20:
+        assert count("pinned") == 1 and count("host copies") > 1
+        break
+    assert (count("host copies"), count("pinned")) == (1, 0), k
+assert k == 19 if storage == "F64" else k == (4 << 20) // out.nbytes
 """)
 
 
-@pytest.mark.parametrize("storage,shape,copies", [("F64", (64, 64, 65), 1), ("F32", (64, 64, 65), 2), ("F32", (8, 4, 4), 1)])
-def test_field_copy_without_pinned_memory(child, storage, shape, copies):
-    """No pinned memory to be had: one pageable copy of values that go as they
-    are, chunks of a million values where they are widened."""
-    child(FIELD + "storage, shape, copies = %r, %r, %r" % (storage, shape, copies) + """
+@pytest.mark.parametrize("storage,pinned", [("F64", 0), ("F64", 1), ("F32", 0)])
+def test_large_field_copies(child, storage, pinned):
+    """From 32 MB on (4 MB widened) a field is staged, but for values that go as
+    they are into memory that the device reaches: those take one copy."""
+    child(FIELD + "storage, pinned = %r, %r" % (storage, pinned) + """
+lat, want = field(storage, 128, 128, 65 if storage == "F64" else 33)
+out = np.zeros_like(want)
+if pinned:
+    fake.fake_pinned(out.ctypes.data, out.nbytes)
+read(lat, out)
+np.testing.assert_array_equal(out, want)
+assert count("pinned") == 1 - pinned and (count("host copies") == 1) == bool(pinned)
+assert (fake.fake_last_copy_to() == out.ctypes.data) == bool(pinned)
+""")
+
+
+@pytest.mark.parametrize("storage,shape", [("F64", (128, 128, 65)), ("F32", (128, 128, 33)), ("F32", (3, 1, 1))])
+def test_field_copy_without_pinned_memory(child, storage, shape):
+    """No pinned memory to be had: one pageable copy."""
+    child(FIELD + "storage, shape = %r, %r" % (storage, shape) + """
 lat, want = field(storage, *shape)
 fake.fake_no_pinned(1)
 out = np.zeros_like(want)
 read(lat, out)
 np.testing.assert_array_equal(out, want)
-assert count("host copies") == copies, count("host copies")
+assert count("host copies") == 1
 """)
 
 
@@ -225,7 +245,7 @@ assert count("host copies") == copies, count("host copies")
 def test_field_copy_without_memory_for_a_thread(child, which):
     """No memory for the state of a helper thread: the caller takes its share."""
     child(FIELD + "which = %r" % which + """
-lat, want = field("F32", 64, 64, 64)  # 16 chunks: four threads
+lat, want = field("F32", 128, 64, 64)  # 16 MB to the caller: staged, four threads
 out = np.zeros_like(want)
 fake.fake_fail_new(which)
 read(lat, out)

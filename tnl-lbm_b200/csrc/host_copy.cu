@@ -5,8 +5,6 @@
 #include <cstring>
 #include <exception>
 #include <functional>
-#include <memory>
-#include <new>
 #include <thread>
 
 namespace lbm {
@@ -90,25 +88,20 @@ cudaError_t direct_copy(cudaStream_t stream, const void* dev, void* host, size_t
 	return e == cudaSuccess ? cudaStreamSynchronize(stream) : e;
 }
 
-// without pinned memory: one copy where the values go as they are, else through
-// a buffer of as many values as there is memory for
-cudaError_t pageable_copy(cudaStream_t stream, const void* dev, int dev_size, void* host, int host_size, long long n)
+// floats widened to doubles without staging: one copy into the upper half of the
+// caller's memory, widened there from the front.  Value i ends at byte 8 i + 8, and
+// the next one still waits from 4 n + 4 (i + 1) on: not before that for any i < n.
+cudaError_t widen_in_place(cudaStream_t stream, const void* dev, void* host, long long n)
 {
-	if (dev_size == host_size)
-		return direct_copy(stream, dev, host, (size_t) n * dev_size);
-	float small[4096];
-	const long long many = n < (1 << 20) ? n : 1 << 20;
-	std::unique_ptr<float[]> large(new (std::nothrow) float[(size_t) many]);
-	float* const chunk = large ? large.get() : small;
-	const long long per_chunk = large ? many : 4096;
-	for (long long first = 0; first < n; first += per_chunk) {
-		const long long count = n - first < per_chunk ? n - first : per_chunk;
-		cudaError_t e = cudaMemcpyAsync(chunk, (const float*) dev + first, (size_t) count * sizeof(float), cudaMemcpyDeviceToHost, stream);
-		if (e == cudaSuccess)
-			e = cudaStreamSynchronize(stream);
-		if (e != cudaSuccess)
-			return e;
-		deliver(reinterpret_cast<const unsigned char*>(chunk), dev_size, (unsigned char*) host, host_size, first, count);
+	unsigned char* const floats = (unsigned char*) host + 4 * (size_t) n;
+	const cudaError_t e = direct_copy(stream, dev, floats, 4 * (size_t) n);
+	if (e != cudaSuccess)
+		return e;
+	float part[1024];
+	for (long long first = 0; first < n; first += 1024) {
+		const long long count = n - first < 1024 ? n - first : 1024;
+		std::memcpy(part, floats + 4 * first, 4 * (size_t) count);
+		deliver(reinterpret_cast<const unsigned char*>(part), 4, (unsigned char*) host, 8, first, count);
 	}
 	return cudaSuccess;
 }
@@ -132,8 +125,12 @@ cudaError_t host_copy(HostCopy& c, int device, cudaStream_t stream, const void* 
 {
 	if (n < 1)
 		return cudaStreamSynchronize(stream);
-	if (dev_size == host_size && reached_by_device(host))
-		return direct_copy(stream, dev, host, (size_t) n * dev_size);
+	const bool widen = dev_size != host_size;
+	const size_t bytes = (size_t) n * host_size;
+	if (!widen && (bytes < HostCopy::STAGE_COPIES || reached_by_device(host)))
+		return direct_copy(stream, dev, host, bytes);
+	if (!c.pinned && widen && (c.unstaged += bytes) < HostCopy::STAGE_WIDENED)
+		return widen_in_place(stream, dev, host, n);
 	if (!c.pinned) {
 		cudaError_t e = cudaMallocHost((void**) &c.pinned, 2 * HostCopy::THREADS * HostCopy::CHUNK);
 		for (cudaEvent_t& ev : c.landed)
@@ -143,7 +140,7 @@ cudaError_t host_copy(HostCopy& c, int device, cudaStream_t stream, const void* 
 			// no pinned memory to be had
 			host_copy_free(c);
 			cudaGetLastError();
-			return pageable_copy(stream, dev, dev_size, host, host_size, n);
+			return widen ? widen_in_place(stream, dev, host, n) : direct_copy(stream, dev, host, bytes);
 		}
 	}
 	Job j;
