@@ -25,10 +25,10 @@ namespace lbm {
 // (OUT) needs no more registers than the plain step: its outputs are written
 // before the collision.  The FP64 kernels need twice the registers per value.
 //
-// FP64 arithmetic: 4 blocks (128 registers, at most 48 bytes of spills).  With the
-// warp sync between loads and collision (aa_step_site) the kernels take 110-142
-// registers; without it 168 and spills, at 3 blocks for SRT, BGK and the
-// Geier-2017 cumulant.  B200, us a step: Taylor-Green vortex (Geier 2017) 64^3 18.0
+// FP64 arithmetic: 4 blocks (128 registers, at most 48 bytes of spills, 100 in
+// SRT's odd step without a map).  With the warp sync between loads and collision
+// (aa_step_site) the kernels take 110-142 registers; without it 168 and spills, at
+// 3 blocks for SRT, BGK and the Geier-2017 cumulant.  B200, us a step: Taylor-Green vortex (Geier 2017) 64^3 18.0
 // -> 16.6, 128^3 154.5 -> 146.1; duct 256x96x96 SRT 159 -> 155, BGK 162 -> 155,
 // cumulant and MRT 155 (432 bytes a site through HBM at 6.6 TB/s).
 template <typename R, int COLL, int CUMF, bool ODD, bool GENERAL, bool OUT>
@@ -52,9 +52,9 @@ constexpr int ade_minb()
 }
 
 // resident blocks of the A-B step; its FP32 observation variant spills at 5.
-// FP64 as the A-A step, with the same warp sync (168 registers and 56-144 bytes
-// of spills without it, at 3 blocks): duct 256x96x96 cumulant 166.6 -> 154.5 us a
-// step.
+// FP64 with the A-A step's warp sync at 4 blocks (504-568 bytes of spills, which L1
+// takes) instead of 3 without it (168 registers, 56-144 bytes): duct 256x96x96
+// cumulant 166.6 -> 154.5 us a step, 432 bytes a site through HBM at 6.6 TB/s.
 template <typename R, int COLL, int CUMF, bool OUT>
 constexpr int ab_minb()
 {

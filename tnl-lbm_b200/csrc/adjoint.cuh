@@ -33,16 +33,16 @@ namespace lbm {
 // Resident blocks per SM of the adjoint step (register cap 65536 / (128 n)).  It
 // moves 520 bytes a site (27 FP64 values in and out, 4 moments, the force, the
 // force gradient in and out) and is bound by the latency of its gathers: 64 steps
-// of a 160x48x48 channel backward took 2597 us at 4 blocks, 2512 at 5, 2497 at 6
-// (80 registers, 44 bytes of spills in the odd step), against 6599 when each step
+// of a 160x48x48 channel backward take 2598 us at 4 blocks, 2520 at 5, 2490 at 6
+// (80 registers, 44 bytes of spills in the odd step), against 6595 when each step
 // read the 27 primal populations, summed direction by direction and ran on rows
 // of 128 threads.
 #ifndef ADJ_STEP_MINB
 #define ADJ_STEP_MINB 6
 #endif
-// and of the primal step with a force field: 64 steps forward (FP32) took
-// 2180 us at 4 blocks, 2207 at 5 (92-112 bytes of spills), 2320 at 6; FP64
-// spills 330 bytes at 4 and runs 3
+// and of the primal step with a force field: the 64 steps forward (FP32, moments
+// kept) take 1700 us at 4 blocks, 1740 at 5 (92-112 bytes of spills), 1850 at 6
+// (2330 with checkpoints instead of moments); FP64 spills 330 bytes at 4 and runs 3
 #ifndef ADJ_PRIMAL_MINB
 #define ADJ_PRIMAL_MINB 4
 #endif

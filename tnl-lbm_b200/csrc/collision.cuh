@@ -45,7 +45,9 @@ enum : int
 	EQ_INV_CUM = 1
 };
 
-// per-lattice constants of the collision slot, in the compute type
+// Per-lattice constants of the collision slot, in the compute type.  w1_3, w3 ..
+// w5, c43 and cB are left for the collisions of plugins: the built-in ones read
+// what is folded from them (l3 .. l5, kA, k45, kB).
 template <typename R>
 struct CollParams
 {

@@ -223,10 +223,12 @@ int ensure_lanes(lbm_ensemble e)
 
 // Members are independent of one another, so a block of steps runs group by
 // group: the populations of a group of small members stay in L2 from step to
-// step instead of passing through HBM once per step.  Members in order, a group
-// closed when the next member would take it past ENS_GROUP_BYTES (a member
-// larger than that is a group of its own, which costs it nothing) unless it
-// would leave a group too small to fill the GPU.  B200 (126 MB of L2), us a step
+// step instead of passing through HBM once per step.  The members, in order, are
+// cut into about total / ENS_GROUP_BYTES groups of equal shares.  A group is
+// closed ahead of a member more than half of which would lie past its share, once
+// it holds half a share; so it may exceed the share by half a member, and a large
+// member (of which L2 keeps nothing in any case) takes smaller ones into its group
+// that were less than half a share.  B200 (126 MB of L2), us a step
 // for groups of 24, 32, 48, 64, 96 MB and one group: 128 members of 16-32 sites a
 // side 88, 85, 81, 79, 89, 89 (one site per thread); 512 of 16-32 319, 345, 294,
 // 288, 366, 383 and 64 of 32-128 1069, 1066, 1056, 1062, 1093, 1163 (two sites).
@@ -245,7 +247,6 @@ void build_groups(lbm_ensemble e)
 		bytes[m] = 27 * line * g.Y * g.Z;
 		total += bytes[m];
 	}
-	// equal shares of the whole
 	const long long n = (total + ENS_GROUP_BYTES - 1) / ENS_GROUP_BYTES;
 	const long long share = (total + n - 1) / n;
 	long long acc = 0;
@@ -260,8 +261,9 @@ void build_groups(lbm_ensemble e)
 }
 
 // grid policy 2: every member runs the single-lattice step (the two-site
-// kernel where it applies, else the direct kernel) on its lane; the lanes fork from and join into the ensemble's stream, so under
-// graph capture the members become independent branches
+// kernel where it applies, else the direct kernel) on its lane; the lanes fork
+// from and join into the ensemble's stream, so under graph capture the members
+// become independent branches
 int ens_launch_members(lbm_ensemble e, long long iteration)
 {
 	if (int rc = ensure_lanes(e))
@@ -283,7 +285,7 @@ int ens_launch_members(lbm_ensemble e, long long iteration)
 		L.grid = dim3((g.X + bx - 1) / bx, (g.Y + L.block.y - 1) / L.block.y, g.Z);
 		L.stream = e->lanes[m % nl];
 		L.kernel = lbm::KERNEL_DIRECT;
-		// the two-site kernel where it applies (FP32 arithmetic, even X)
+		// the two-site kernel where it applies (FP32 arithmetic)
 		cudaError_t err = cudaErrorNotSupported;
 		if (const lbm::PairStepFn pair = lbm::pair_step_of(e->storage))
 			err = pair(L);

@@ -104,11 +104,11 @@ cudaError_t finish_sums(const double* partials, long long nslots, double* stage,
 						double mass_offset)
 {
 	// programmatic dependent launch: where the finish follows the kernel that
-	// wrote the partials on the same stream, its grid is scheduled while that
-	// kernel's last blocks run (the observation step kernels trigger it when
-	// they start) and waits in griddepcontrol.wait; after a wait on another
-	// stream's event (the sums of lbm_step, on the finish stream) it starts as
-	// an ordinary launch
+	// wrote the partials on the same stream and that kernel lets its dependents
+	// go, its grid is scheduled while the last blocks run and waits in
+	// griddepcontrol.wait; after a wait on another stream's event (the sums of
+	// lbm_step, on the finish stream) or a kernel that does not (the enstrophy's),
+	// it starts as an ordinary launch
 	cudaLaunchConfig_t cfg = {};
 	cfg.gridDim = dim3(FINISH_BLOCKS);
 	cfg.blockDim = dim3(FINISH_THREADS);

@@ -730,7 +730,7 @@ __device__ __forceinline__ void rest_update(const StepArgs<typename S::T, float>
 }
 
 // One A-A step of a lattice without a map, two sites per thread: block b takes
-// pairs b T .. b T + T - 1 of the linear order (T = 64 or 128 threads).
+// pairs b T .. b T + T - 1 of the linear order (T = 32 to 128 threads).
 template <typename S, typename C, bool ODD, bool OUT, bool RAGGED, int MINB>
 __global__ void __launch_bounds__(128, MINB) aa_pair_kernel(const StepArgs<typename S::T, float> a, const CollParams<F2> p2,
 															 const PairSlots ps, const PairRows pr, long long red_slots)
