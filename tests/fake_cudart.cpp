@@ -20,7 +20,7 @@ std::map<std::string, long long> counts;
 std::string trace;	// kernels launched since fake_reset, one a line
 size_t in_use = 0, limit = 0;
 long long launch_to_fail = 0, news_armed = 0;
-bool no_pinned = false;
+bool no_pinned = false, busy = false;
 const char *pinned_first = nullptr, *pinned_last = nullptr;
 const void* last_copy_to = nullptr;
 thread_local cudaError_t last_error = cudaSuccess;
@@ -101,6 +101,10 @@ void fake_limit(size_t bytes)  // of device memory, 0: none
 void fake_fail_launch(long long n)	// the n-th launch from here fails
 {
 	launch_to_fail = n;
+}
+void fake_busy(int on)	// streams are at work when asked
+{
+	busy = on;
 }
 void fake_no_pinned(int on)
 {
@@ -321,6 +325,10 @@ cudaError_t cudaStreamSynchronize(cudaStream_t)
 		news_armed = 0;
 	}
 	return cudaSuccess;
+}
+cudaError_t cudaStreamQuery(cudaStream_t)
+{
+	return busy ? give(cudaErrorNotReady) : cudaSuccess;
 }
 cudaError_t cudaStreamWaitEvent(cudaStream_t, cudaEvent_t, unsigned)
 {

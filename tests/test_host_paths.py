@@ -196,7 +196,7 @@ def read(lat, out):
 def test_field_copies_of_a_new_lattice(child, storage):
     """The first read-outs of a lattice pay for no staging: values that go as they
     are take one copy below 32 MB, values to be widened are copied into the
-    caller's memory and widened there, until 4 MB have gone that way."""
+    caller's memory and widened there, until 16 MB have gone that way."""
     child(FIELD + "storage = %r" % storage + """
 lat, want = field(storage, 33, 32, 31)  # 1 MB
 for k in range(20):
@@ -204,17 +204,35 @@ for k in range(20):
     fake.fake_reset()
     read(lat, out)
     np.testing.assert_array_equal(out, want)
-    if storage == "F32" and (k + 1) * out.nbytes >= 4 << 20:
+    if storage == "F32" and (k + 1) * out.nbytes >= 16 << 20:
         assert count("pinned") == 1 and count("host copies") > 1
         break
     assert (count("host copies"), count("pinned")) == (1, 0), k
-assert k == 19 if storage == "F64" else k == (4 << 20) // out.nbytes
+assert k == 19 if storage == "F64" else k == (16 << 20) // out.nbytes
+""")
+
+
+@pytest.mark.parametrize("storage,shape,staged", [("F32", (33, 32, 31), 0), ("F32", (64, 64, 32), 1), ("F64", (64, 64, 32), 0)])
+def test_field_copies_ahead_of_work(child, storage, shape, staged):
+    """While the stream is at work, staging is made for 4 MB to be widened."""
+    child(FIELD + "storage, shape, staged = %r, %r, %r" % (storage, shape, staged) + """
+lat, want = field(storage, *shape)
+fake.fake_busy(1)
+out = np.zeros_like(want)
+read(lat, out)
+np.testing.assert_array_equal(out, want)
+assert count("pinned") == staged and (count("host copies") > 1) == bool(staged)
+fake.fake_busy(0)
+read(lat, out)
+np.testing.assert_array_equal(out, want)
+assert count("pinned") == staged
+lat.get_populations()  # and the query has left no error behind
 """)
 
 
 @pytest.mark.parametrize("storage,pinned", [("F64", 0), ("F64", 1), ("F32", 0)])
 def test_large_field_copies(child, storage, pinned):
-    """From 32 MB on (4 MB widened) a field is staged, but for values that go as
+    """From 32 MB on (16 MB widened) a field is staged, but for values that go as
     they are into memory that the device reaches: those take one copy."""
     child(FIELD + "storage, pinned = %r, %r" % (storage, pinned) + """
 lat, want = field(storage, 128, 128, 65 if storage == "F64" else 33)

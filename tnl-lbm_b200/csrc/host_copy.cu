@@ -82,6 +82,14 @@ bool reached_by_device(const void* host)
 	return a.type != cudaMemoryTypeUnregistered;
 }
 
+bool at_work(cudaStream_t stream)
+{
+	const cudaError_t e = cudaStreamQuery(stream);
+	if (e != cudaSuccess)
+		cudaGetLastError();	 // not ready, or an error that the copy reports
+	return e == cudaErrorNotReady;
+}
+
 cudaError_t direct_copy(cudaStream_t stream, const void* dev, void* host, size_t bytes)
 {
 	const cudaError_t e = cudaMemcpyAsync(host, dev, bytes, cudaMemcpyDeviceToHost, stream);
@@ -129,7 +137,8 @@ cudaError_t host_copy(HostCopy& c, int device, cudaStream_t stream, const void* 
 	const size_t bytes = (size_t) n * host_size;
 	if (!widen && (bytes < HostCopy::STAGE_COPIES || reached_by_device(host)))
 		return direct_copy(stream, dev, host, bytes);
-	if (!c.pinned && widen && (c.unstaged += bytes) < HostCopy::STAGE_WIDENED)
+	if (!c.pinned && widen && (c.unstaged += bytes) < HostCopy::STAGE_WIDENED
+		&& (bytes < HostCopy::STAGE_BUSY || !at_work(stream)))
 		return widen_in_place(stream, dev, host, n);
 	if (!c.pinned) {
 		cudaError_t e = cudaMallocHost((void**) &c.pinned, 2 * HostCopy::THREADS * HostCopy::CHUNK);
